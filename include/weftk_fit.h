@@ -70,12 +70,13 @@ typedef struct WeftFitState {
     int32_t* sel;            /* [n_tiles * cap_max] selected slot indices (pool-local) */
     /* candidates (slot-indexed) */
     const WeftPrim* cand;    /* [n_slots] candidate records */
-    float* prep;             /* [n_slots * 16] prepared per-candidate terms (64 B each) */
+    float* prep;             /* not used (may be NULL): candidates are prepared where they are scored */
     uint8_t* alive;          /* [n_slots] 1 = still in the pool */
     uint8_t* kind;           /* [n_slots] primitive kind of the slot (filled by prepare / re-seed) */
     float* partial;          /* [n_slots * 4] per-1024-pixel-block squared-error sums (scratch) */
     int32_t* status;         /* [4] round counters: evaluated tiles, improved tiles */
-    unsigned long long* work; /* [2] running totals: candidate-pixels scored, algorithmic FP32 ops
+    unsigned long long* work; /* [2] running totals: candidate-pixels scored (candidates that cannot win
+                                 are not), algorithmic FP32 ops
                                  (per candidate-pixel: per-kind op count + 9 for the error); may be NULL */
     /* Scoring-kernel shape per tile-size class [8-px, 16-px, 32/64-px tiles], an index into
      * that class's table (0 = default; WEFTK_FIT_VARIANTS per class, see weftk_fit_variant):
@@ -117,7 +118,7 @@ typedef struct WeftFitItem {
 } WeftFitItem;
 
 /* Prepare candidate slots [pool_off[t] + lo, pool_off[t] + pool_cnt[t]) of every
- * tile whose slot range changed: compute the prepared terms and mark them live.
+ * tile whose slot range changed: note their kinds and mark them live.
  * first_new[t] = first pool-local slot to prepare (pass pool_cnt[t] to skip). */
 int weftk_fit_prepare(const WeftFitState* st, const int32_t* d_first_new, void* stream);
 

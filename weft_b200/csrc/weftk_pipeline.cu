@@ -85,8 +85,8 @@ struct WeftRefiner {
     DevBuf img, qwork, qtiles;
     // tile-sized (capacity ncap tiles): int32 state, doubles, selections, rows
     DevBuf tint, tdbl, tsel, trows;
-    // slot-sized (ncap * STRIDE): records, prepared terms, flags, partial sums, slot order
-    DevBuf cand, prep, alive, kind, partial, perm;
+    // slot-sized (ncap * STRIDE): records, flags, partial sums, slot order
+    DevBuf cand, alive, kind, partial, perm;
     // pixel-sized: tile pixels and the composite
     DevBuf src4, bg;
     // per-image layout upload and the scoring queue
@@ -124,7 +124,7 @@ extern "C" int weftk_refiner_create(const WeftRefineParams* params, WeftRefiner*
 
 extern "C" int weftk_refiner_destroy(WeftRefiner* r) {
     if (!r) return WEFTK_OK;
-    for (DevBuf* b : {&r->img, &r->qwork, &r->qtiles, &r->tint, &r->tdbl, &r->tsel, &r->trows, &r->cand, &r->prep,
+    for (DevBuf* b : {&r->img, &r->qwork, &r->qtiles, &r->tint, &r->tdbl, &r->tsel, &r->trows, &r->cand,
                       &r->alive, &r->kind, &r->partial, &r->perm, &r->src4, &r->bg, &r->layout, &r->queue, &r->misc})
         if (b->p) cudaFree(b->p);
     for (HostBuf* b : {&r->h_qt, &r->h_layout})
@@ -304,7 +304,6 @@ extern "C" int weftk_refine_image(WeftRefiner* r, const uint8_t* h_img, int h, i
         if ((rc = grow(r->tdbl, (size_t)nc * 7 * sizeof(double)))) return rc;  // cur_obj, moments x6
         if ((rc = grow(r->trows, (size_t)nc * (4 * 16 + 1) * sizeof(float)))) return rc;  // p, m, v, q, loss
         if ((rc = grow(r->cand, (size_t)nc * STRIDE * sizeof(WeftPrim)))) return rc;
-        if ((rc = grow(r->prep, (size_t)nc * STRIDE * 16 * sizeof(float)))) return rc;
         if ((rc = grow(r->alive, (size_t)nc * STRIDE))) return rc;
         if ((rc = grow(r->kind, (size_t)nc * STRIDE))) return rc;
         if ((rc = grow(r->partial, (size_t)nc * STRIDE * 4 * sizeof(float)))) return rc;
@@ -389,7 +388,6 @@ extern "C" int weftk_refine_image(WeftRefiner* r, const uint8_t* h_img, int h, i
     st.cur_obj = cur_obj;
     st.sel = static_cast<int32_t*>(r->tsel.p);
     st.cand = static_cast<const WeftPrim*>(r->cand.p);
-    st.prep = static_cast<float*>(r->prep.p);
     st.alive = static_cast<uint8_t*>(r->alive.p);
     st.kind = static_cast<uint8_t*>(r->kind.p);
     st.partial = static_cast<float*>(r->partial.p);

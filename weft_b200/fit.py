@@ -222,7 +222,6 @@ class BatchedFit:
         self.t_flags = torch.zeros(n, dtype=torch.int32, device=d)
         self.t_cur_obj = torch.zeros(n, dtype=torch.float64, device=d)
         self.t_sel = torch.full((n * self.cap_max,), -1, dtype=torch.int32, device=d)
-        self.t_prep = torch.empty(self.n_slots * 16, dtype=torch.float32, device=d)
         self.t_alive = torch.zeros(self.n_slots, dtype=torch.uint8, device=d)
         self.t_kind = torch.zeros(self.n_slots, dtype=torch.uint8, device=d)
         self.t_partial = torch.empty(self.n_slots * 4, dtype=torch.float32, device=d)
@@ -234,7 +233,7 @@ class BatchedFit:
             n, self.cap_max, self.n_slots,
             *[_lib.ptr(x) for x in (self.t_src, self.t_bg, self.t_px_off, self.t_size, self.t_cap, self.t_pool_off,
                                     self.t_pool_cnt, self.t_pool_cap, self.t_n_alive, self.t_n_sel, self.t_sel_bits,
-                                    self.t_flags, self.t_cur_obj, self.t_sel, self.t_cand, self.t_prep, self.t_alive,
+                                    self.t_flags, self.t_cur_obj, self.t_sel, self.t_cand, None, self.t_alive,
                                     self.t_kind, self.t_partial, self.t_status, self.t_work)])
         self.stats = FitStats()
         self.device_reseeded = False
