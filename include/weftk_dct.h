@@ -61,17 +61,6 @@ int weftk_dct_apply(const WeftDctTile* d_tiles, int n_tiles, const int16_t* d_co
                     float* d_image, int width, int height, int clip_all, void* stream);
 
 /*
- * The same layer over tiles listed by class in one launch: group g is the `count[g]` tiles from
- * d_tiles + first[g], none larger than sides[g] (a power of two in 4..64; the lists are host
- * arrays, n_groups <= WEFTK_DCT_MAX_GROUPS).  weftk_dct_apply is this with one group.
- */
-#define WEFTK_DCT_MAX_GROUPS 8
-int weftk_dct_layer(const WeftDctTile* d_tiles, int n_groups, const int32_t* sides, const int32_t* first,
-                    const int32_t* count, const int16_t* d_coeffs, int64_t n_coeffs, int chroma_mode,
-                    int band_layout, float quant_step, float freq_alpha, float* d_image, int width, int height,
-                    int clip_all, void* stream);
-
-/*
  * Raster resize of the decoder: d_src (src_h x src_w x 3 float32) -> u8 = trunc(clip(x * 255,
  * 0, 255)) -> Pillow BILINEAR resize to dst_w x dst_h -> d_dst = u8 / 255 (float32, HWC).
  * d_tmp: caller scratch of src_h * dst_w * 3 bytes (the horizontal pass of large downscales; other sizes

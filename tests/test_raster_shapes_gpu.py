@@ -1,5 +1,5 @@
 """The raster branch at the sizes where its kernels change course: a DCT layer's classes of tiles
-(partly filled CTAs, every side, the classes in one launch and tiles smaller than their class), and
+(partly filled CTAs, every side, launches that follow one another, tiles smaller than their class), and
 the resize's window in shared memory (widths with and without four-wide stores, one-pixel sides,
 downscales that take fewer rows per CTA and ones that fall back to two kernels)."""
 
@@ -42,13 +42,13 @@ def _run(descs, coeffs, groups, chroma, band, image):
     lib = _lib.lib_for_device(0)
     td = torch.from_numpy(descs.view(np.uint8)).cuda()
     tc = torch.from_numpy(coeffs).cuda()
-    lists = [np.array(v, np.int32) for v in zip(*groups)]
     st = ctypes.c_int(0)
     lib.weftk_device_status(ctypes.addressof(st))
-    rc = lib.weftk_dct_layer(_lib.ptr(td), len(groups), _lib.ptr(lists[0]), _lib.ptr(lists[1]), _lib.ptr(lists[2]),
-                             _lib.ptr(tc), len(coeffs), chroma, band, 0.02, 4.0, _lib.ptr(image),
-                             int(image.shape[1]), int(image.shape[0]), 0, torch.cuda.current_stream().cuda_stream)
-    assert rc == 0
+    for side, first, count in groups:
+        rc = lib.weftk_dct_apply(_lib.ptr(td) + first * descs.itemsize, count, _lib.ptr(tc), len(coeffs), chroma, band,
+                                 0.02, 4.0, side, _lib.ptr(image), int(image.shape[1]), int(image.shape[0]), 0,
+                                 torch.cuda.current_stream().cuda_stream)
+        assert rc == 0
     _lib.check(lib.weftk_device_status(ctypes.addressof(st)), "weftk_device_status")
     assert st.value == 0
     return image

@@ -1,7 +1,7 @@
 // weftk_dct.cu — the decoder's raster branch: per-tile DCT residual layer and the u8 BILINEAR
 // resize (see include/weftk_dct.h).
 //
-// DCT layer: one launch over every tile side, a CTA per 4096 pixels of one side's tiles.  Each channel's
+// DCT layer: a launch per tile side, a CTA per 4096 pixels of its tiles.  Each channel's
 // quantized block is gathered straight from the coefficient stream (tile-major or band-major zigzag: the
 // band-to-tile permutation is only an address computation), dequantized and inverse-transformed in
 // float64 as two separable passes through shared memory, rounded to float32; the three channels are then
@@ -65,8 +65,8 @@ __global__ void dct_tables_kernel() {
 }
 
 // The layer's kernel: 256 threads take 4096 pixels' worth of tiles of one side's class (one tile of 64,
-// 64 tiles of 8), so a launch over all classes is a few hundred equal CTAs, two per SM, the long ones
-// (64 px) first.  A thread owns a 4 x 4 set of a block's outputs, rows and columns n / 4 apart, so that
+// 64 tiles of 8), so the classes of a picture are a few hundred equal CTAs, two per SM; the launches of the
+// classes overlap (a launch may start beside the one before it).  A thread owns a 4 x 4 set of a block's outputs, rows and columns n / 4 apart, so that
 // neighbouring lanes read and write neighbouring columns; per step of a pass it reads 4 + 4 values for 16
 // float64 multiply-adds.  Cb and Cr of 4:2:0 go together, a quarter of the threads each.  Quantisation
 // steps depend on u + v only and are tabulated per CTA.
@@ -81,14 +81,9 @@ static_assert(256 * dct_slot_words(4) <= kDctBlockWords && 64 * dct_slot_words(8
               "every class's blocks fit");
 constexpr size_t kDctSmem = (2 * kDctBlockWords + 2 * kDctSteps) * sizeof(double) + 2 * DC_PIXELS * sizeof(float);
 
-struct DctGroups {  // classes of tiles, in launch order
-    int n;
-    int log_side[WEFTK_DCT_MAX_GROUPS], first[WEFTK_DCT_MAX_GROUPS], count[WEFTK_DCT_MAX_GROUPS];
-    int unit0[WEFTK_DCT_MAX_GROUPS + 1];  // first CTA
-};
-
 struct DctLayer {
     const WeftDctTile* tiles;
+    int n_tiles, log_side;  // the class: no tile is larger
     const int16_t* coeffs;
     long long n_coeffs;
     int chroma, band;
@@ -162,7 +157,7 @@ __device__ __forceinline__ void dct_cols(const double* __restrict__ A, const dou
 
 // HALF: 4:2:0 (chroma mode 2)
 template <bool HALF>
-__global__ void __launch_bounds__(DC_THREADS, 2) dct_layer_kernel(DctLayer L, DctGroups G) {
+__global__ void __launch_bounds__(DC_THREADS, 2) dct_layer_kernel(DctLayer L) {
     extern __shared__ double dct_smem[];
     double* X = dct_smem;                     // dequantized blocks [slot][u * pitch + v]
     double* T = X + kDctBlockWords;           // after the pass along v: [slot][u * pitch + x]
@@ -172,14 +167,15 @@ __global__ void __launch_bounds__(DC_THREADS, 2) dct_layer_kernel(DctLayer L, Dc
     double* basis = reinterpret_cast<double*>(R);
     constexpr int R_PLANE = HALF ? DC_PIXELS / 4 : DC_PIXELS;
     const int tid = threadIdx.x;
-    int g = 0;
-    while (g + 1 < G.n && (int)blockIdx.x >= G.unit0[g + 1]) ++g;
-    const int LS = G.log_side[g];             // the class: tiles of side 2^LS (or below)
+    // the launch that follows may be the layer's next class: it can start beside this one, and does its
+    // transforms, but waits for this one (below) before it touches the image
+    asm volatile("griddepcontrol.launch_dependents;");
+    const int LS = L.log_side;
     const int log_slots = 12 - 2 * LS, log_tpt = 2 * LS - 4;  // slots * threads per tile = 256
     const int slot_words = dct_slot_words(1 << LS);
-    const int tile0 = ((int)blockIdx.x - G.unit0[g]) << log_slots;
-    const WeftDctTile* tiles = L.tiles + G.first[g] + tile0;
-    const int n_slots = min(1 << log_slots, G.count[g] - tile0);
+    const int tile0 = (int)blockIdx.x << log_slots;
+    const WeftDctTile* tiles = L.tiles + tile0;
+    const int n_slots = min(1 << log_slots, L.n_tiles - tile0);
 
     auto side_ok = [&](int S) { return S >= 4 && S <= (1 << LS) && (S & (S - 1)) == 0; };
     for (int i = tid; i < 2 * kDctSteps; i += DC_THREADS) {
@@ -325,6 +321,7 @@ __global__ void __launch_bounds__(DC_THREADS, 2) dct_layer_kernel(DctLayer L, Dc
     }
     __syncthreads();
 
+    asm volatile("griddepcontrol.wait;" ::: "memory");  // the image as the launches before leave it
     const int nb = S >> 2;
     if (S == 0 || lt >= nb * nb) return;
     const WeftDctTile* tp = tiles + slot;
@@ -683,50 +680,40 @@ int grid_for(long long total) {
 
 using namespace weftk;
 
-extern "C" int weftk_dct_layer(const WeftDctTile* d_tiles, int n_groups, const int32_t* sides, const int32_t* first,
-                               const int32_t* count, const int16_t* d_coeffs, int64_t n_coeffs, int chroma_mode,
-                               int band_layout, float quant_step, float freq_alpha, float* d_image, int width,
-                               int height, int clip_all, void* stream) {
+extern "C" int weftk_dct_apply(const WeftDctTile* d_tiles, int n_tiles, const int16_t* d_coeffs, int64_t n_coeffs,
+                               int chroma_mode, int band_layout, float quant_step, float freq_alpha, int max_size,
+                               float* d_image, int width, int height, int clip_all, void* stream) {
     static_assert(sizeof(WeftDctTile) == 64, "WeftDctTile must be 64 bytes");
-    WEFTK_REQUIRE(n_groups >= 0 && n_groups <= WEFTK_DCT_MAX_GROUPS && n_coeffs >= 0, "dct_layer: bad count");
-    WEFTK_REQUIRE(n_groups == 0 || (sides && first && count), "dct_layer: null group list");
-    WEFTK_REQUIRE(chroma_mode >= 0 && chroma_mode <= 2, "dct_layer: chroma_mode must be 0, 1 or 2");
-    WEFTK_REQUIRE(band_layout == 0 || band_layout == 1, "dct_layer: layout must be 0 or 1");
-    WEFTK_REQUIRE(width > 0 && height > 0 && d_image, "dct_layer: bad image");
-    WEFTK_REQUIRE(!(freq_alpha < 0.0f), "dct_layer: freq_alpha must be >= 0");
-    DctGroups G = {};
-    long long units = 0;
-    for (int side = WEFTK_DCT_MAX_TILE; side >= 1; side >>= 1) {  // the long ones first
-        for (int g = 0; g < n_groups; ++g) {
-            if (sides[g] != side || count[g] == 0) continue;
-            WEFTK_REQUIRE(side >= 4 && first[g] >= 0 && count[g] > 0, "dct_layer: bad group");
-            int log_side = 0;
-            while ((1 << log_side) < side) ++log_side;
-            G.log_side[G.n] = log_side;
-            G.first[G.n] = first[g];
-            G.count[G.n] = count[g];
-            G.unit0[G.n] = (int)units;
-            units += ceil_div(count[g], DC_PIXELS / (side * side));
-            WEFTK_REQUIRE(units <= 0x7fffffff, "dct_layer: too many tiles");
-            ++G.n;
-        }
-    }
-    int listed = 0;
-    for (int g = 0; g < n_groups; ++g) listed += count[g] != 0;
-    WEFTK_REQUIRE(listed == G.n, "dct_layer: a group's side must be a power of two in 4..64");
-    G.unit0[G.n] = (int)units;
+    WEFTK_REQUIRE(n_tiles >= 0 && n_coeffs >= 0, "dct_apply: negative count");
+    WEFTK_REQUIRE(chroma_mode >= 0 && chroma_mode <= 2, "dct_apply: chroma_mode must be 0, 1 or 2");
+    WEFTK_REQUIRE(band_layout == 0 || band_layout == 1, "dct_apply: layout must be 0 or 1");
+    WEFTK_REQUIRE(width > 0 && height > 0 && d_image, "dct_apply: bad image");
+    WEFTK_REQUIRE(max_size >= 4 && max_size <= WEFTK_DCT_MAX_TILE && (max_size & (max_size - 1)) == 0,
+                  "dct_apply: max_size must be a power of two in 4..64");
+    WEFTK_REQUIRE(!(freq_alpha < 0.0f), "dct_apply: freq_alpha must be >= 0");
     cudaStream_t s = (cudaStream_t)stream;
-    if (units > 0) {
-        WEFTK_REQUIRE(d_tiles && (d_coeffs || n_coeffs == 0), "dct_layer: null pointer");
+    if (n_tiles > 0) {
+        WEFTK_REQUIRE(d_tiles && (d_coeffs || n_coeffs == 0), "dct_apply: null pointer");
         int rc = ensure_tables(s);
         if (rc != WEFTK_OK) return rc;
         auto kernel = chroma_mode == 2 ? dct_layer_kernel<true> : dct_layer_kernel<false>;
         WEFTK_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kDctSmem));
         const double step = (double)quant_step;
-        const DctLayer L = {d_tiles,    d_coeffs, (long long)n_coeffs, chroma_mode, band_layout, step,
-                            step * 1.5, (double)freq_alpha, d_image, width, height};
-        kernel<<<(unsigned)units, DC_THREADS, kDctSmem, s>>>(L, G);
-        WEFTK_CUDA(cudaGetLastError());
+        int log_side = 2;
+        while ((1 << log_side) < max_size) ++log_side;
+        const DctLayer L = {d_tiles, n_tiles, log_side, d_coeffs, (long long)n_coeffs, chroma_mode, band_layout,
+                            step, step * 1.5, (double)freq_alpha, d_image, width, height};
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3((unsigned)ceil_div(n_tiles, DC_PIXELS / (max_size * max_size)));
+        cfg.blockDim = dim3(DC_THREADS);
+        cfg.dynamicSmemBytes = kDctSmem;
+        cfg.stream = s;
+        cudaLaunchAttribute attr = {};
+        attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr.val.programmaticStreamSerializationAllowed = 1;
+        cfg.attrs = &attr;
+        cfg.numAttrs = 1;
+        WEFTK_CUDA(cudaLaunchKernelEx(&cfg, kernel, L));
     }
     if (clip_all) {
         const long long n = (long long)width * height * 3;
@@ -734,17 +721,6 @@ extern "C" int weftk_dct_layer(const WeftDctTile* d_tiles, int n_groups, const i
         WEFTK_CUDA(cudaGetLastError());
     }
     return WEFTK_OK;
-}
-
-extern "C" int weftk_dct_apply(const WeftDctTile* d_tiles, int n_tiles, const int16_t* d_coeffs, int64_t n_coeffs,
-                               int chroma_mode, int band_layout, float quant_step, float freq_alpha, int max_size,
-                               float* d_image, int width, int height, int clip_all, void* stream) {
-    WEFTK_REQUIRE(n_tiles >= 0 && n_coeffs >= 0, "dct_apply: negative count");
-    WEFTK_REQUIRE(max_size >= 4 && max_size <= WEFTK_DCT_MAX_TILE && (max_size & (max_size - 1)) == 0,
-                  "dct_apply: max_size must be a power of two in 4..64");
-    const int32_t side = max_size, first = 0, count = n_tiles;
-    return weftk_dct_layer(d_tiles, 1, &side, &first, &count, d_coeffs, n_coeffs, chroma_mode, band_layout, quant_step,
-                           freq_alpha, d_image, width, height, clip_all, stream);
 }
 
 extern "C" int weftk_raster_resize(const float* d_src, int src_w, int src_h, float* d_dst, int dst_w, int dst_h,

@@ -10,7 +10,7 @@ Here the host only parses the block and turns the presence mask, per-tile scales
 coefficient layout (tile-major, or band-major zigzag, src/weft/dct_residual.py:221-296) into
 one 64-byte descriptor per tile holding each channel's coefficient base and stride; the
 gather, dequantization, inverse DCT, colour transform, add and clip run in
-``weftk_dct_layer``, the resize in ``weftk_raster_resize``.  Errors follow the reference's:
+``weftk_dct_apply``, the resize in ``weftk_raster_resize``.  Errors follow the reference's:
 a malformed block raises ``ValueError``.
 """
 
@@ -161,8 +161,8 @@ def tile_table(block: DctBlock, quad_tiles, width: int, height: int, scales=None
 
 class DctLaunch:
     """A BLOCK_DCT bound to a tile list and an image size, with its descriptors and coefficients
-    resident on the device; ``run`` enqueues the layer (one launch over all tile sides, then the
-    whole-image clip) without host synchronisation."""
+    resident on the device; ``run`` enqueues the layer (one ``weftk_dct_apply`` launch per tile
+    side, then the whole-image clip) without host synchronisation."""
 
     def __init__(self, block: DctBlock, quad_tiles, width: int, height: int, device: int = 0, scales=None):
         import torch
@@ -178,7 +178,6 @@ class DctLaunch:
         sizes = self.descs["size"]
         self.groups = [(int(v), int(np.searchsorted(sizes, v, "left")), int(np.searchsorted(sizes, v, "right")))
                        for v in np.unique(sizes)]
-        self.group_lists = np.array([[s, lo, hi - lo] for s, lo, hi in self.groups], np.int32).reshape(-1, 3).T.copy()
 
     @classmethod
     def from_payload(cls, payload: bytes, quad_tiles, width: int, height: int, device: int = 0) -> "DctLaunch":
@@ -186,7 +185,7 @@ class DctLaunch:
 
     @property
     def launches(self) -> int:
-        return 2 if self.groups else 1
+        return len(self.groups) + 1
 
     def flops(self) -> float:
         """Float64 operations of the two transform passes: 2 n^3 multiply-adds per n x n block."""
@@ -195,12 +194,15 @@ class DctLaunch:
 
     def run(self, image, stream: int, clip_all: bool = True) -> None:
         b = self.block
-        g = self.group_lists
-        _lib.check(self.lib.weftk_dct_layer(_lib.ptr(self.t_descs) if self.groups else 0, len(self.groups),
-                                            _lib.ptr(g[0]), _lib.ptr(g[1]), _lib.ptr(g[2]),
-                                            _lib.ptr(self.t_coeffs), int(b.coeffs.size), b.chroma_mode, b.layout,
-                                            b.quant_step, b.freq_alpha, _lib.ptr(image), self.width, self.height,
-                                            int(bool(clip_all)), stream), "weftk_dct_layer")
+        for s, lo, hi in self.groups:
+            _lib.check(self.lib.weftk_dct_apply(_lib.ptr(self.t_descs) + lo * DCT_TILE_DTYPE.itemsize, hi - lo,
+                                                _lib.ptr(self.t_coeffs), int(b.coeffs.size), b.chroma_mode, b.layout,
+                                                b.quant_step, b.freq_alpha, s, _lib.ptr(image), self.width,
+                                                self.height, 0, stream), "weftk_dct_apply")
+        if clip_all:
+            _lib.check(self.lib.weftk_dct_apply(0, 0, 0, 0, b.chroma_mode, b.layout, b.quant_step, b.freq_alpha, 4,
+                                                _lib.ptr(image), self.width, self.height, 1, stream),
+                       "weftk_dct_apply")
 
 
 def apply_dct(image, payload: bytes, quad_tiles, clip_all: bool = True):
