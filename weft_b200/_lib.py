@@ -57,6 +57,13 @@ class WeftStackSet(ctypes.Structure):
         ("kinds_mask", ctypes.c_int32), ("moments", ctypes.c_void_p)]
 
 
+class WeftSceneFile(ctypes.Structure):
+    """A file in host memory and where its parts stand (include/weftk_entropy.h)."""
+    _fields_ = [("blob", ctypes.c_void_p)] + [
+        (n, ctypes.c_int64) for n in ("blob_len", "prim", "prim_len", "cidx", "toc", "qtree", "res0", "res1")] + [
+        (n, ctypes.c_int32) for n in ("n_chunks", "n_tiles", "n_res1", "enc_w", "enc_h", "out_w", "out_h", "_pad")]
+
+
 class WeftRefineParams(ctypes.Structure):
     """Parameters of a per-image refiner (include/weftk_pipeline.h)."""
     _fields_ = [("cap", ctypes.c_int32), ("steps", ctypes.c_int32), ("min_tile", ctypes.c_int32),
@@ -107,6 +114,7 @@ SIGNATURES: dict[str, list] = {
     "weftk_fit_reset": [_P, _P, _P],
     "weftk_build_residuals": [_P, _P, _I, _P, _P, _I, _P, _P, _P],
     "weftk_fit_moments": [_P, _P, _P],
+    "weftk_decode_scene": [_P, _P, _I, _P, _P],
     "weftk_rans_decode_chunks": [_P, ctypes.c_int64, _P, _I, _P, ctypes.c_int64, _P],
     "weftk_fit_run": [_P, _I, ctypes.c_double, ctypes.c_double, _P, _P, _I, _P, _I, _P, _I, _P, _P],
     "weftk_refine_start": [_P, _P, _I, _P, _P, _P, _P, _P],

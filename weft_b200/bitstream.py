@@ -313,9 +313,8 @@ def ctypes_addr_of(v) -> int:
     return ctypes.addressof(v)
 
 
-def decode_weft(blob: bytes, device: int | None = None) -> WeftFile:
-    """Parse a WEFT file; with ``device`` the PRIM chunks are entropy-decoded on that GPU.
-    A malformed file raises ``BitstreamError``."""
+def _directory(blob: bytes):
+    """Block spans (tag -> (offset, length)) and the HEAD fields, checked in the reference's order."""
     if len(blob) < 12:
         raise BitstreamError("truncated file header")
     magic, major, minor, n_blocks, _ = struct.unpack_from("<4sBBHI", blob, 0)
@@ -325,29 +324,93 @@ def decode_weft(blob: bytes, device: int | None = None) -> WeftFile:
         raise BitstreamError(f"unsupported major version: {major}")
     if 12 + 20 * n_blocks > len(blob):
         raise BitstreamError("truncated block directory")
-    blocks = {}
+    spans = {}
     off = 12
     for _ in range(n_blocks):
         tag, b_off, b_len = struct.unpack_from("<4sQQ", blob, off)
         off += 20
         if b_off + b_len > len(blob):
             raise BitstreamError("block extends past EOF")
-        blocks[tag] = blob[b_off:b_off + b_len]
+        spans[tag] = (b_off, b_len)
     for tag in (b"HEAD", b"TOC ", b"PRIM", b"META", b"QTRE"):
-        if tag not in blocks:
+        if tag not in spans:
             raise BitstreamError(f"missing required block: {tag.decode('ascii').strip()}")
-    for tag in blocks:
-        if blocks[tag][:4] == b"\x28\xb5\x2f\xfd":
+    for b_off, b_len in spans.values():
+        if blob[b_off:b_off + min(b_len, 4)] == b"\x28\xb5\x2f\xfd":
             raise BitstreamError("zstd-compressed blocks are not supported")
-    if len(blocks[b"HEAD"]) != struct.calcsize("<IIHHBBHIIBBH"):
+    if spans[b"HEAD"][1] != struct.calcsize("<IIHHBBHIIBBH"):
         raise BitstreamError("invalid HEAD size")
-    w, h, ts, mp, _cs, _qm, flags, _tc, _tr, quality, _pid, _ = struct.unpack("<IIHHBBHIIBBH", blocks[b"HEAD"])
+    head = struct.unpack_from("<IIHHBBHIIBBH", blob, spans[b"HEAD"][0])
+    w, h, ts, mp = head[:4]
     if w <= 0 or h <= 0:
         raise BitstreamError("invalid dimensions")
     if ts <= 0 or ts > 64:
         raise BitstreamError("invalid tile size")
     if mp <= 0 or mp > 255:
         raise BitstreamError("invalid max primitives")
+    return spans, head
+
+
+def scene_layout(blob):
+    """``(_lib.WeftSceneFile without its bytes and target size, DCT payload or None, width, height)`` of a file of
+    the form ``encode_weft`` writes (chunked PRIM, one RES0 and quadtree entry per tile, 4x4 RES1 grids),
+    for the decode on the device; None for any other, which ``decode_weft`` reads or refuses."""
+    from . import _lib
+
+    if not isinstance(blob, bytes):
+        return None
+    try:
+        spans, head = _directory(blob)
+        flags = head[6]
+        if b"CIDX" not in spans or ((flags & FLAG_HAS_DCT) and b"DCT " not in spans):
+            return None
+
+        def u32(tag):
+            if spans[tag][1] < 4:
+                raise BitstreamError("truncated block")
+            return struct.unpack_from("<I", blob, spans[tag][0])[0]
+
+        n_toc, n_chunks, n_tree = u32(b"TOC "), u32(b"CIDX"), u32(b"QTRE")
+        n = n_toc - 1
+        if (n <= 0 or spans[b"TOC "][1] != 4 + 4 * n_toc or spans[b"CIDX"][1] < 4 + 24 * n_chunks or
+                n_tree != n or spans[b"QTRE"][1] < 4 + 5 * n_tree):
+            return None
+        res0 = res1 = -1
+        n_res1 = 0
+        if b"RES0" in spans:
+            n_res0 = u32(b"RES0")
+            if n_res0 < n or spans[b"RES0"][1] < 4 + 3 * n_res0:
+                return None
+            res0 = spans[b"RES0"][0] + 4
+        if b"RES1" in spans:
+            if spans[b"RES1"][1] < 8:
+                return None
+            n_res1, gw, gh, _ = struct.unpack_from("<IBBH", blob, spans[b"RES1"][0])
+            if (gw, gh) != (4, 4) or spans[b"RES1"][1] < 8 + 48 * n_res1:
+                return None
+            res1 = spans[b"RES1"][0] + 8
+        m_off, m_len = spans[b"META"]
+        meta = json.loads(blob[m_off + 4:m_off + m_len].decode())
+        ew, eh = int(meta.get("encode_width", head[0])), int(meta.get("encode_height", head[1]))
+        if not (0 < ew < 1 << 30 and 0 < eh < 1 << 30):
+            return None
+    except (ValueError, TypeError, AttributeError, OverflowError, struct.error):
+        return None
+    f = _lib.WeftSceneFile(None, len(blob), *spans[b"PRIM"], spans[b"CIDX"][0] + 4, spans[b"TOC "][0] + 4,
+                           spans[b"QTRE"][0] + 4, res0, res1, n_chunks, n, n_res1, ew, eh)
+    dct = None
+    if b"DCT " in spans:
+        d_off, d_len = spans[b"DCT "]
+        dct = blob[d_off:d_off + d_len]
+    return f, dct, head[0], head[1]
+
+
+def decode_weft(blob: bytes, device: int | None = None) -> WeftFile:
+    """Parse a WEFT file; with ``device`` the PRIM chunks are entropy-decoded on that GPU.
+    A malformed file raises ``BitstreamError``."""
+    spans, head = _directory(blob)
+    blocks = {tag: blob[b_off:b_off + b_len] for tag, (b_off, b_len) in spans.items()}
+    w, h, ts, mp, _cs, _qm, flags, _tc, _tr, quality, _pid, _ = head
     toc_b = blocks[b"TOC "]
     if len(toc_b) < 4:
         raise BitstreamError("truncated TOC")

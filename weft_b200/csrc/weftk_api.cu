@@ -9,6 +9,7 @@
 #include <vector>
 
 #include "weftk_common.cuh"
+#include "weftk_scene.cuh"
 
 static_assert(sizeof(WeftPrim) == 60, "WeftPrim must match the reference's 60-byte PrimData");
 static_assert(sizeof(WeftEval) == 16, "WeftEval must match the reference's EvalDesc");
@@ -18,7 +19,7 @@ namespace weftk {
 
 int launch_score_evals(const WeftEval*, int, const WeftPrim*, const float*, float*, int, cudaStream_t);
 int launch_render_tiles(const WeftTileDecodeDesc*, int, const int2*, int, const WeftPrim*, const float*, int,
-                        const float*, int, float*, int, int, cudaStream_t);
+                        const float*, int, float*, int, int, cudaStream_t, const int* d_n_items = nullptr);
 int read_device_status(int* status, bool clear);
 
 static thread_local std::string t_last_error;
@@ -226,6 +227,55 @@ int weftk_render_tiles_host(const WeftTileDecodeDesc* h_descs, int n_tiles, cons
     WEFTK_CUDA(cudaMemcpyAsync(h_out, dout, out_bytes, cudaMemcpyDeviceToHost, s));
     WEFTK_CUDA(cudaStreamSynchronize(s));
     return check_status_after_sync();
+}
+
+int weftk_decode_scene(const WeftSceneFile* file, float* out, int on_device, int* irregular, void* stream) {
+    WEFTK_REQUIRE(file && file->blob && out && irregular, "decode_scene: null pointer");
+    *irregular = 1;
+    const WeftSceneFile& f = *file;
+    ScenePlan plan;
+    int rc = scene_plan(f, plan);
+    if (rc || !plan.ok) return rc;
+    std::lock_guard<std::mutex> lock(g_arena_mu);
+    Arena* a = nullptr;
+    if ((rc = arena_for_current(&a))) return rc;
+    const size_t out_bytes = sizeof(float) * 3 * (size_t)f.out_h * (size_t)f.out_w;
+    void *dblob, *dchunks, *draw, *dd, *dp, *dc, *dr, *di, *dctl, *dout = out;
+    if ((rc = arena_get(10, (size_t)f.blob_len, &dblob, *a))) return rc;
+    if ((rc = arena_get(11, sizeof(WeftRansChunk) * plan.chunks.size(), &dchunks, *a))) return rc;
+    if ((rc = arena_get(12, (size_t)plan.raw_len, &draw, *a))) return rc;
+    if ((rc = arena_get(13, 2 * sizeof(int), &dctl, *a))) return rc;
+    if ((rc = arena_get(4, sizeof(WeftTileDecodeDesc) * (size_t)f.n_tiles, &dd, *a))) return rc;
+    if ((rc = arena_get(5, sizeof(WeftPrim) * (size_t)plan.cap_prims, &dp, *a))) return rc;
+    if ((rc = arena_get(6, sizeof(float) * 48 * (size_t)plan.cap_cp48, &dc, *a))) return rc;
+    if ((rc = arena_get(7, sizeof(float) * 48 * (size_t)std::max(1, f.n_res1), &dr, *a))) return rc;
+    if ((rc = arena_get(9, sizeof(int2) * (size_t)std::max(1, plan.n_items), &di, *a))) return rc;
+    if (!on_device && (rc = arena_get(8, out_bytes, &dout, *a))) return rc;
+    cudaStream_t s = on_device ? (cudaStream_t)stream : a->stream;
+    const SceneBuffers b = {(const uint8_t*)dblob,    (const WeftRansChunk*)dchunks, (uint8_t*)draw,
+                            (WeftTileDecodeDesc*)dd,  (WeftPrim*)dp,                 (float*)dc,
+                            (float*)dr,               (int2*)di,                     (int*)dctl};
+    WEFTK_CUDA(cudaMemcpyAsync(dblob, f.blob, (size_t)f.blob_len, cudaMemcpyHostToDevice, s));
+    WEFTK_CUDA(cudaMemcpyAsync(dchunks, plan.chunks.data(), sizeof(WeftRansChunk) * plan.chunks.size(),
+                               cudaMemcpyHostToDevice, s));
+    int ctl[2] = {0, 0};
+    rc = scene_launch(f, plan, b, s);
+    if (!rc) {
+        WEFTK_CUDA(cudaMemsetAsync(dout, 0, out_bytes, s));
+        const int n_res1 = std::min(f.n_res1, f.n_tiles);
+        rc = launch_render_tiles(b.descs, f.n_tiles, b.items, plan.n_items, b.prims, b.cp48, plan.cap_cp48,
+                                 n_res1 ? b.grids : nullptr, n_res1, (float*)dout, f.out_h, f.out_w, s, b.ctl + 1);
+    }
+    if (!rc) {
+        WEFTK_CUDA(cudaMemcpyAsync(ctl, dctl, sizeof(ctl), cudaMemcpyDeviceToHost, s));
+        if (!on_device) WEFTK_CUDA(cudaMemcpyAsync(out, dout, out_bytes, cudaMemcpyDeviceToHost, s));
+    }
+    // (the arena's buffers and the chunk list are this call's until its work is done)
+    const cudaError_t e = cudaStreamSynchronize(s);
+    if (rc) return rc;
+    WEFTK_CUDA(e);
+    *irregular = ctl[0] != 0;
+    return WEFTK_OK;
 }
 
 }  // extern "C"

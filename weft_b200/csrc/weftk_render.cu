@@ -536,7 +536,8 @@ __device__ __forceinline__ void render_item(const int2 item, const WeftTileDecod
 __global__ void __launch_bounds__(DEC_THREADS, DEC_MINB) render_tiles_kernel(
     const WeftTileDecodeDesc* __restrict__ descs, int n_tiles, const int2* __restrict__ items, int n_items,
     const WeftPrim* __restrict__ prims, const float* __restrict__ cp48, int n_cp48, const float* __restrict__ res1,
-    int n_res1, float* __restrict__ out, int H, int W) {
+    int n_res1, float* __restrict__ out, int H, int W, const int* __restrict__ n_items_dev) {
+    if (n_items_dev) n_items = min(n_items, *n_items_dev);  // counted on the device, at most n_items
     __shared__ Prep sp_all[DEC_WARPS][MAX_TILE_PRIMS];
     __shared__ float grid_all[DEC_WARPS][48];
     __shared__ float ctrl_all[DEC_WARPS][48];
@@ -596,7 +597,7 @@ int launch_score_evals(const WeftEval* d_evals, int n_evals, const WeftPrim* d_p
 
 int launch_render_tiles(const WeftTileDecodeDesc* d_descs, int n_tiles, const int2* d_items, int n_items,
                         const WeftPrim* d_prims, const float* d_cp48, int n_cp48, const float* d_res1, int n_res1,
-                        float* d_out, int out_h, int out_w, cudaStream_t stream) {
+                        float* d_out, int out_h, int out_w, cudaStream_t stream, const int* d_n_items) {
     if (n_tiles == 0) return WEFTK_OK;
     WEFTK_REQUIRE(n_tiles > 0 && d_descs && d_out && out_h > 0 && out_w > 0, "render_tiles: bad arguments");
     WEFTK_REQUIRE(n_cp48 >= 0 && n_res1 >= 0, "render_tiles: negative table size");
@@ -607,7 +608,7 @@ int launch_render_tiles(const WeftTileDecodeDesc* d_descs, int n_tiles, const in
     WEFTK_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
     const int blocks = std::min((n_items + DEC_WARPS - 1) / DEC_WARPS, sms * DEC_MINB);
     render_tiles_kernel<<<blocks, DEC_THREADS, 0, stream>>>(d_descs, n_tiles, d_items, n_items, d_prims, d_cp48,
-                                                            n_cp48, d_res1, n_res1, d_out, out_h, out_w);
+                                                            n_cp48, d_res1, n_res1, d_out, out_h, out_w, d_n_items);
     WEFTK_CUDA(cudaGetLastError());
     return WEFTK_OK;
 }

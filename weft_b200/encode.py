@@ -11,11 +11,12 @@ decoded file (src/weft/encoder.py:3926-3931, :4008-4011).
 
 from __future__ import annotations
 
+import ctypes
 from dataclasses import dataclass
 
 import numpy as np
 
-from . import bitstream, rate, render
+from . import _lib, bitstream, rate, render
 from .candidates import Cand
 
 
@@ -70,7 +71,52 @@ def encode_fit(width, height, quality, tiles, patches, stacks, recon, with_res0=
 def decode_file(blob: bytes, target_width=None, target_height=None) -> np.ndarray:
     """Decode a primitive-stack WEFT file with the GPU decoder walk (linear float32 RGB); the target
     defaults to the file's width and height.  A file with a DCT residual block takes the raster
-    branch: walk at the encoded size, DCT residual, u8 BILINEAR resize to the target."""
+    branch: walk at the encoded size, DCT residual, u8 BILINEAR resize to the target.
+
+    A file of the ordinary form is entropy-decoded, parsed and rendered on the device
+    (``weftk_decode_scene``); any other goes through the host parser below, which also raises for a
+    malformed one."""
+    scene = bitstream.scene_layout(blob)
+    if scene is not None:
+        out = _decode_on_device(blob, scene, target_width, target_height)
+        if out is not None:
+            return out
+    return _decode_general(blob, target_width, target_height)
+
+
+def _decode_on_device(blob: bytes, scene, target_width, target_height):
+    """``decode_file`` of a laid-out file, or None where the general path has to judge it."""
+    f, dct, width, height = scene
+    tw, th = int(target_width or width), int(target_height or height)
+    if not (0 < tw < 1 << 30 and 0 < th < 1 << 30):
+        return None
+    data = np.frombuffer(blob, np.uint8)
+    f.blob = _lib.ptr(data)
+    f.out_w, f.out_h = (tw, th) if dct is None else (f.enc_w, f.enc_h)
+    lib = _lib.lib_for_device(0)
+    irregular = ctypes.c_int(0)
+
+    def run(out, on_device, stream):
+        _lib.check(lib.weftk_decode_scene(ctypes.addressof(f), _lib.ptr(out), on_device,
+                                          ctypes.addressof(irregular), stream), "weftk_decode_scene")
+        return None if irregular.value else out
+
+    if dct is None:
+        return run(np.empty((th, tw, 3), np.float32), 0, 0)
+    import torch
+
+    from . import raster
+
+    img = torch.empty((f.enc_h, f.enc_w, 3), dtype=torch.float32, device="cuda:0")
+    if run(img, 1, torch.cuda.current_stream(img.device).cuda_stream) is None:
+        return None
+    rows = np.frombuffer(blob, np.uint8, 5 * f.n_tiles, f.qtree).reshape(-1, 5).astype(np.int64)
+    qtree = np.stack([rows[:, 0] + 256 * rows[:, 1], rows[:, 2] + 256 * rows[:, 3], rows[:, 4]], 1).tolist()
+    img = raster.apply_dct(img, dct, [tuple(t) for t in qtree])
+    return raster.resize(img, tw, th).cpu().numpy()
+
+
+def _decode_general(blob: bytes, target_width=None, target_height=None) -> np.ndarray:
     wf = bitstream.decode_weft(blob)
     tiles = [type("QT", (), {"x": x, "y": y, "size": s})() for x, y, s in wf.qtree]
     stacks = bitstream.decode_tiles(wf.prim_raw, wf.toc)
