@@ -5,9 +5,9 @@
 // composites the whole stack for them in registers; the per-lane squared error of a
 // chunk is summed in float32 and accumulated in float64; one warp reduction per eval.
 //
-// Decode walk: work items of tile rows, one warp per item, a persistent one-wave grid.
-// Lone constant tiles (almost every tile of a fit at q75) are written as whole 16-byte
-// slots of their rows, other tiles per 4-pixel group with the stack composited in
+// Decode walk: work items of tile rows, one warp per item.  Two kernels run side by side: one
+// for lone constant tiles (almost every tile of a fit at q75), which are written as runs of
+// their rows, and one for all others, per 4-pixel group with the stack composited in
 // registers.  Output is float32 HWC.
 #include <cuda_runtime.h>
 
@@ -142,21 +142,31 @@ __device__ __noinline__ void bicubic_pixel(const float* ctrl, int lx, int ly, in
 // first primitive, one item per lane), so the dependent-load chain item -> descriptor
 // -> primitive is paid once per batch instead of once per item.
 //
-// Three ways to write an item's rows:
-//  * a lone constant layer without a RES1 grid is one colour: every lane stores whole
-//    16-byte slots of the row's float run (slot s holds channels s, s+1, s+2, s mod 3 of
-//    the colour), so a warp's stores are contiguous and fill every 32-byte sector they
-//    touch; the at most three floats at each end of a row that share a slot with the
-//    neighbouring tile are stored one by one;
-//  * a lone constant layer with a RES1 grid: the same 16-byte slots, each the colour plus
-//    the bilinear grid at its two pixels (no primitive evaluation);
-//  * anything else: per 4-pixel group, the whole stack composited in registers.
+// Two kernels walk the same list.  Both take the whole list's records, so that neither
+// needs a second list; each leaves the other's items.
+//  * render_fill_kernel: lone constant layers, with or without a RES1 grid, at 64 registers.
+//    What an item needs (clipped rect, final colour, grid) is worked out by one lane per item
+//    of the batch, and the stores are runs of the rows: where rows are 16-byte aligned, whole
+//    16-byte slots (slot s holds channels s, s+1, s+2, s mod 3 of the colour), the at most
+//    three floats at each end of a row that share a slot with the neighbouring tile one by
+//    one; else one float per lane.  Either way a warp's stores are contiguous.
+//  * render_tiles_kernel: anything else, per 4-pixel group, at twice the registers.  A CTA
+//    looks through 128 items at once and its four warps share those that are its own, 32 groups in
+//    turn: one warp on a whole item of four layers needs 40 us, whatever the others do.
 // Which tile writes a pixel, and with what arithmetic, is the same on every path, so the
 // image does not depend on the order or the path the items take.
+// Bound: the stores' bandwidth where few tiles are evaluated per pixel.  1024 x 1024 fitted
+// tiles, 1 in 17 evaluated, into 3840 x 2160 take 38 us (99.5 MB: 15 us), and 57 with both sorts in one
+// kernel, whose 127 registers left 11 warps a SM to the fills; 1919 x 1079 with RES1 grids, whose rows
+// are not aligned, take 27 us, and 55 with four pixels a lane and 12 strided stores for each.  With four
+// layers in every tile, 3840 x 2160, 184 us, and 230 with a warp to an item; 24 layers, 1024 x 1024,
+// 141 and 144.
 constexpr int DEC_ITEM_GROUPS = WEFTK_DECODE_ITEM_GROUPS;
 constexpr int DEC_WARPS = DEC_THREADS / 32;
+static_assert((DEC_WARPS & (DEC_WARPS - 1)) == 0, "steps are dealt out modulo DEC_WARPS");
 constexpr int DEC_MINB = 4;  // resident CTAs per SM the register budget is set for
 constexpr int DEC_BATCH = 8;
+constexpr int FILL_MINB = 8;  // the same for the fill kernel
 
 __device__ __forceinline__ int floor_div4(int v) { return v >= 0 ? (v >> 2) : -((-v + 3) >> 2); }
 
@@ -311,14 +321,75 @@ __device__ __forceinline__ void fill_rows_res1(float* __restrict__ out, size_t r
     }
 }
 
+// The same two fills where rows are not 16-byte aligned: a lane per float of the rows' runs, the same
+// column (so the same pixel and channel) in every row it walks.
+__device__ __forceinline__ void fill_rows_any(float* __restrict__ out, size_t row_floats, int gy0, int r0, int r1,
+                                              int xa, int xb, float c0, float c1, float c2, int lane) {
+    const int n = 3 * (xb - xa), per_row = n < 32 ? n : 32, rs = n < 32 ? 32 / n : 1;
+    const int rr = lane / per_row, cl = lane - rr * per_row;
+    if (rr >= rs || r0 + rr >= r1) return;
+    for (int c = cl; c < n; c += per_row) {
+        const float v = sel3(c % 3, c0, c1, c2);
+        float* dst = out + (size_t)(gy0 + r0 + rr) * row_floats + 3 * xa + c;
+        for (int r = r0 + rr; r < r1; r += rs, dst += rs * row_floats) *dst = v;
+    }
+}
+
+__device__ __forceinline__ void fill_rows_res1_any(float* __restrict__ out, size_t row_floats, int gy0, int r0, int r1,
+                                                   int x0, int w, int xa, int xb, float gscale,
+                                                   const float* __restrict__ grid, float c0, float c1, float c2,
+                                                   int lane) {
+    const int n = 3 * (xb - xa), per_row = n < 32 ? n : 32, rs = n < 32 ? 32 / n : 1;
+    const int rr = lane / per_row, cl = lane - rr * per_row;
+    if (rr >= rs || r0 + rr >= r1) return;
+    for (int c = cl; c < n; c += per_row) {
+        const int px = c / 3, ch = c - 3 * px;
+        const float base = sel3(ch, c0, c1, c2);
+        int a0, a1, ry_cached = -1;
+        float wx, top = 0.0f, bot = 0.0f;
+        res1_axis(min(max(xa + px - x0, 0), w - 1), gscale, a0, a1, wx);
+        float* dst = out + (size_t)(gy0 + r0 + rr) * row_floats + 3 * xa + c;
+        for (int r = r0 + rr; r < r1; r += rs, dst += rs * row_floats) {
+            int ry0, ry1;
+            float wy;
+            res1_axis(r, gscale, ry0, ry1, wy);
+            if (ry0 != ry_cached) {
+                ry_cached = ry0;
+                top = lerp_rn(grid[(ry0 * 4 + a0) * 3 + ch], grid[(ry0 * 4 + a1) * 3 + ch], wx);
+                bot = lerp_rn(grid[(ry1 * 4 + a0) * 3 + ch], grid[(ry1 * 4 + a1) * 3 + ch], wx);
+            }
+            *dst = clamp01(base + lerp_rn(top, bot, wy));
+        }
+    }
+}
+
 __device__ __forceinline__ bool desc_ok(const WeftTileDecodeDesc& d) {
     return d.prim_count >= 0 && d.prim_count <= MAX_TILE_PRIMS && d.target_w > 0 && d.target_h > 0 &&
            d.target_w <= 8192 && d.target_h <= 8192 && d.source_size > 0;
 }
 
+// The item's rows [r0, r1) and columns [xa, xb) inside the image; false when there are none.
+__device__ __forceinline__ bool item_rect(const int2 item, const WeftTileDecodeDesc& d, int H, int W, int& r0, int& r1,
+                                          int& xa, int& xb) {
+    const int G = floor_div4(d.target_x0 + d.target_w + 3) - floor_div4(d.target_x0);  // aligned groups per row
+    r0 = max(item.y, -d.target_y0);
+    r1 = min(min(d.target_h, item.y + max(1, DEC_ITEM_GROUPS / G)), H - d.target_y0);
+    xa = max(d.target_x0, 0);
+    xb = min(d.target_x0 + d.target_w, W);
+    return r0 < r1 && xa < xb;
+}
+
+// render_fill_kernel's items: a lone constant layer; its RES1 index, if it has one, inside the table
+__device__ __forceinline__ bool fill_item(const WeftTileDecodeDesc& d, int kind0, const float* res1, int n_res1) {
+    return desc_ok(d) && d.prim_count == 1 && kind0 == K_CONST &&
+           !(res1 != nullptr && n_res1 > 0 && d.res1_index >= n_res1);
+}
+
 // One work item (tile rows) rendered by one warp; p0 is the tile's first primitive (unset
-// when the tile has none); sp / grid / ctrl are the warp's shared-memory slices.
-__device__ __forceinline__ void render_item(const int2 item, const WeftTileDecodeDesc& d, const WeftPrim& p0,
+// when the tile has none), prepared, and geo its sampling step and RES1 scale; sp / grid / ctrl are the
+// warp's shared-memory slices.  The warp
+// takes steps part, part + DEC_WARPS, .. of the item, 32 groups each; returns how many steps it has.
+__device__ __forceinline__ int render_item(const int2 item, int part, const WeftTileDecodeDesc& d, const Prep& p0, float2 geo,
                                             const WeftPrim* __restrict__ prims, const float* __restrict__ cp48,
                                             int n_cp48, const float* __restrict__ res1, int n_res1,
                                             float* __restrict__ out, int H, int W, bool w_aligned, size_t row_floats,
@@ -326,120 +397,40 @@ __device__ __forceinline__ void render_item(const int2 item, const WeftTileDecod
     const int n = d.prim_count, w = d.target_w, h = d.target_h;
     if (!desc_ok(d)) {
         if (lane == 0) report(WEFTK_E_ARG);
-        return;
+        return 0;
     }
     const int a0 = floor_div4(d.target_x0);
     const int G = floor_div4(d.target_x0 + w + 3) - a0;  // aligned groups per row
-    // the item's rows, cropped to the image
-    const int r0 = max(item.y, -d.target_y0);
-    const int r1 = min(min(h, item.y + max(1, DEC_ITEM_GROUPS / G)), H - d.target_y0);
-    const int xa = max(d.target_x0, 0), xb = min(d.target_x0 + w, W);
-    if (r0 >= r1 || xa >= xb) return;  // nothing of this item is inside the image
+    int r0, r1, xa, xb;
+    if (!item_rect(item, d, H, W, r0, r1, xa, xb)) return 0;  // nothing of this item is inside the image
     const bool has_res1 = res1 != nullptr && n_res1 > 0 && d.res1_index >= 0;
     if (has_res1 && d.res1_index >= n_res1) {
         if (lane == 0) report(WEFTK_E_ARG);
-        return;
+        return 0;
     }
-    if (n == 1 && !has_res1 && w_aligned && p0.kind == K_CONST) {
-        // a lone constant layer: the blend over black and the RES0 add, once per item
-        const Prep c = prep_prim(p0);
-        fill_rows(out, row_floats, d.target_y0, r0, r1, xa, xb,
-                  clamp01(blend(c.cr, c.a, 0.0f) + d.res0_r), clamp01(blend(c.cg, c.a, 0.0f) + d.res0_g),
-                  clamp01(blend(c.cb, c.a, 0.0f) + d.res0_b), lane);
-        return;
-    }
-    for (int i = lane; i < n; i += 32)
-        sp[i] = prep_prim(i == 0 ? p0 : load_prim(prims + d.prim_offset + i));
+    const int steps = ((r1 - r0) * G + 31) >> 5;
+    if (part >= steps) return steps;
+    const Prep* stack = n == 1 ? &p0 : sp;
+    if (n > 1)
+        for (int i = lane; i < n; i += 32) sp[i] = i == 0 ? p0 : prep_prim(load_prim(prims + d.prim_offset + i));
     if (has_res1)
         for (int i = lane; i < 48; i += 32) grid[i] = res1[(size_t)d.res1_index * 48 + i];
     __syncwarp();
-    const bool bic = (n == 1 && sp[0].kind == K_BICUBIC);
+    const bool bic = (n == 1 && p0.kind == K_BICUBIC);
     if (bic) {
-        const int gi = (int)sp[0].q[0];
+        const int gi = (int)p0.q[0];
         if (cp48 == nullptr || gi < 0 || gi >= n_cp48) {
             if (lane == 0) report(WEFTK_E_ARG);
-            return;
+            return steps;
         }
         for (int i = lane; i < 48; i += 32) ctrl[i] = cp48[(size_t)gi * 48 + i];
         __syncwarp();
     }
     const int side = max(w, h);
-    const float step = (side == d.source_size) ? 1.0f : (float)((double)d.source_size / (double)side);
-    const float gscale = (float)(4.0 / (double)h);  // RES1 is upsampled at the cropped tile's height
+    const float step = geo.x, gscale = geo.y;
     const int g_end = r1 * G;                           // < 2^24 for any rect the host accepts
     const float invG = 1.0f / (float)G;
-    if (n == 1 && sp[0].kind == K_CONST && w_aligned && has_res1) {
-        // a lone constant layer with a RES1 grid (the grid is staged in shared memory)
-        fill_rows_res1(out, row_floats, d.target_y0, r0, r1, d.target_x0, w, xa, xb, gscale, grid,
-                       clamp01(blend(sp[0].cr, sp[0].a, 0.0f) + d.res0_r),
-                       clamp01(blend(sp[0].cg, sp[0].a, 0.0f) + d.res0_g),
-                       clamp01(blend(sp[0].cb, sp[0].a, 0.0f) + d.res0_b), lane);
-        return;
-    }
-    if (n == 1 && sp[0].kind == K_CONST && has_res1) {
-        // A lone constant layer with a RES1 grid on rows that are not 16-byte aligned: one colour
-        // plus the bilinear grid per pixel.  Each lane steps its group (row, column) by 32 groups
-        // instead of dividing.  (Without a grid such a tile takes the general path below.)
-        const float fr = clamp01(blend(sp[0].cr, sp[0].a, 0.0f) + d.res0_r);
-        const float fg = clamp01(blend(sp[0].cg, sp[0].a, 0.0f) + d.res0_g);
-        const float fb = clamp01(blend(sp[0].cb, sp[0].a, 0.0f) + d.res0_b);
-        const int x0 = d.target_x0, x1 = d.target_x0 + w;
-        const int drow = 32 / G, dcol = 32 - drow * G;
-        int row = r0 + lane / G, col = lane - (lane / G) * G;
-        for (int g = r0 * G + lane; g - lane < g_end; g += 32, row += drow, col += dcol) {
-            if (col >= G) {
-                col -= G;
-                ++row;
-            }
-            if (g >= g_end) continue;
-            const int gy = d.target_y0 + row;
-            const int gxs = (a0 + col) * 4;
-            float* dst = out + (size_t)gy * row_floats + (size_t)gxs * 3;
-            const bool full = w_aligned && gxs >= x0 && gxs + DEC_PPL <= x1 && gxs >= 0 && gxs + DEC_PPL <= W;
-            float o[DEC_PPL][3];
-            // Bilinear 4x4 grid at pixel centres, edge-clamped (src/weft/render.py:474-515).
-            const float gyf =
-                fminf(fmaxf(__fsub_rn(__fmul_rn((float)row + 0.5f, gscale), 0.5f), 0.0f), 3.0f);
-            const int ry0 = (int)floorf(gyf), ry1 = min(ry0 + 1, 3);
-            const float wy = __fsub_rn(gyf, (float)ry0);
-#pragma unroll
-            for (int j = 0; j < DEC_PPL; ++j) {
-                const int lxc = min(max(gxs + j - x0, 0), w - 1);
-                const float gx =
-                    fminf(fmaxf(__fsub_rn(__fmul_rn((float)lxc + 0.5f, gscale), 0.5f), 0.0f), 3.0f);
-                const int rx0 = (int)floorf(gx), rx1 = min(rx0 + 1, 3);
-                const float wx = __fsub_rn(gx, (float)rx0);
-                const float base[3] = {fr, fg, fb};
-#pragma unroll
-                for (int ch = 0; ch < 3; ++ch) {
-                    const float c00 = grid[(ry0 * 4 + rx0) * 3 + ch], c01 = grid[(ry0 * 4 + rx1) * 3 + ch];
-                    const float c10 = grid[(ry1 * 4 + rx0) * 3 + ch], c11 = grid[(ry1 * 4 + rx1) * 3 + ch];
-                    const float top = __fadd_rn(__fmul_rn(c00, __fsub_rn(1.0f, wx)), __fmul_rn(c01, wx));
-                    const float bot = __fadd_rn(__fmul_rn(c10, __fsub_rn(1.0f, wx)), __fmul_rn(c11, wx));
-                    o[j][ch] = clamp01(base[ch] + __fadd_rn(__fmul_rn(top, __fsub_rn(1.0f, wy)),
-                                                            __fmul_rn(bot, wy)));
-                }
-            }
-            if (full) {
-                float4* d4 = reinterpret_cast<float4*>(dst);
-                d4[0] = make_float4(o[0][0], o[0][1], o[0][2], o[1][0]);
-                d4[1] = make_float4(o[1][1], o[1][2], o[2][0], o[2][1]);
-                d4[2] = make_float4(o[2][2], o[3][0], o[3][1], o[3][2]);
-                continue;
-            }
-#pragma unroll
-            for (int j = 0; j < DEC_PPL; ++j) {
-                const int gxp = gxs + j;
-                if (gxp >= x0 && gxp < x1 && gxp >= 0 && gxp < W) {
-                    dst[3 * j] = o[j][0];
-                    dst[3 * j + 1] = o[j][1];
-                    dst[3 * j + 2] = o[j][2];
-                }
-            }
-        }
-        return;
-    }
-    for (int g0 = r0 * G; g0 < g_end; g0 += 32) {
+    for (int g0 = r0 * G + 32 * part; g0 < g_end; g0 += 32 * DEC_WARPS) {
         const int g = g0 + lane;
         const bool g_ok = g < g_end;
         // row = g / G via the float reciprocal, corrected by one step (exact for g < 2^24)
@@ -471,7 +462,7 @@ __device__ __forceinline__ void render_item(const int2 item, const WeftTileDecod
             }
         } else {
             for (int k = 0; k < n; ++k) {
-                Prep pr = sp[k];
+                Prep pr = stack[k];
                 if (pr.kind == K_BICUBIC) pr.kind = K_SKIP;  // kind 5 inside a longer stack is skipped
                 float a[DEC_PPL], sr[DEC_PPL], sg[DEC_PPL], sb[DEC_PPL];
                 prim_eval<DEC_PPL>(pr, fx, fy, a, sr, sg, sb, lane);
@@ -531,56 +522,148 @@ __device__ __forceinline__ void render_item(const int2 item, const WeftTileDecod
             }
         }
     }
+    return steps;
+}
+
+// round r of warp gw of n_warps: item r * n_warps + gw (r even) or r * n_warps + n_warps - 1 - gw (r odd)
+__device__ __forceinline__ long long item_index(int r, int n_warps, int gw) {
+    return (long long)r * n_warps + ((r & 1) ? n_warps - 1 - gw : gw);
 }
 
 __global__ void __launch_bounds__(DEC_THREADS, DEC_MINB) render_tiles_kernel(
     const WeftTileDecodeDesc* __restrict__ descs, int n_tiles, const int2* __restrict__ items, int n_items,
     const WeftPrim* __restrict__ prims, const float* __restrict__ cp48, int n_cp48, const float* __restrict__ res1,
     int n_res1, float* __restrict__ out, int H, int W, const int* __restrict__ n_items_dev) {
+    asm volatile("griddepcontrol.launch_dependents;");  // render_fill_kernel runs beside this one
     if (n_items_dev) n_items = min(n_items, *n_items_dev);  // counted on the device, at most n_items
     __shared__ Prep sp_all[DEC_WARPS][MAX_TILE_PRIMS];
     __shared__ float grid_all[DEC_WARPS][48];
     __shared__ float ctrl_all[DEC_WARPS][48];
-    __shared__ int2 bitem_all[DEC_WARPS][DEC_BATCH];
-    __shared__ WeftTileDecodeDesc bdesc_all[DEC_WARPS][DEC_BATCH];
-    __shared__ WeftPrim bprim_all[DEC_WARPS][DEC_BATCH];
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    int2* bitem = bitem_all[wid];
-    WeftTileDecodeDesc* bdesc = bdesc_all[wid];
-    WeftPrim* bprim = bprim_all[wid];
+    __shared__ int2 litem[DEC_THREADS];
+    __shared__ WeftTileDecodeDesc ldesc[DEC_THREADS];
+    __shared__ Prep lprep[DEC_THREADS];
+    __shared__ float2 lgeo[DEC_THREADS];
+    __shared__ int listed;
+    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
     const bool w_aligned = (W & 3) == 0 && (reinterpret_cast<uintptr_t>(out) & 15) == 0;
+    const size_t row_floats = (size_t)3 * W;
+    for (int round0 = 0; (long long)round0 * gridDim.x < n_items; round0 += DEC_THREADS) {
+        if (tid == 0) listed = 0;
+        __syncthreads();
+        // the CTA's next items, one per thread: those of this kernel are listed
+        const long long idx = item_index(round0 + tid, gridDim.x, blockIdx.x);
+        if (idx < n_items) {
+            const int2 item = items[idx];
+            if (item.x < 0 || item.x >= n_tiles || item.y < 0) {
+                report(WEFTK_E_ARG);
+            } else {
+                const WeftTileDecodeDesc dd = descs[item.x];
+                const bool prim = desc_ok(dd) && dd.prim_count >= 1;
+                if (!fill_item(dd, prim ? __ldg(&prims[dd.prim_offset].kind) : -1, res1, n_res1)) {
+                    const int k = atomicAdd(&listed, 1);
+                    litem[k] = item;
+                    ldesc[k] = dd;
+                    if (prim) lprep[k] = prep_prim(load_prim(prims + dd.prim_offset));
+                    if (desc_ok(dd)) {
+                        const int side = max(dd.target_w, dd.target_h);
+                        // RES1 is upsampled at the cropped tile's height
+                        lgeo[k] = make_float2(
+                            side == dd.source_size ? 1.0f : (float)((double)dd.source_size / (double)side),
+                            (float)(4.0 / (double)dd.target_h));
+                    }
+                }
+            }
+        }
+        __syncthreads();
+        // the list's steps (32 groups each) go to the warps in turn, whichever item they belong to
+        for (int k = 0, step = 0; k < listed; ++k) {
+            __syncwarp();  // this warp's readers of sp/grid/ctrl from the previous item are done
+            step += render_item(litem[k], (wid - step) & (DEC_WARPS - 1), ldesc[k], lprep[k], lgeo[k], prims, cp48, n_cp48, res1,
+                                n_res1, out, H, W, w_aligned, row_floats, sp_all[wid], grid_all[wid], ctrl_all[wid],
+                                lane);
+        }
+        __syncthreads();
+    }
+}
+
+// An item of the fill kernel, ready to be written.
+struct __align__(16) FillItem {
+    int gy0, r0, r1, xa;
+    int xb, x0, w, grid;  // grid: RES1 index, -1 none
+    float c0, c1, c2, gscale;
+};
+
+template <bool ALIGNED>
+__global__ void __launch_bounds__(DEC_THREADS, FILL_MINB) render_fill_kernel(
+    const WeftTileDecodeDesc* __restrict__ descs, int n_tiles, const int2* __restrict__ items, int n_items,
+    const WeftPrim* __restrict__ prims, const float* __restrict__ res1, int n_res1, float* __restrict__ out, int H,
+    int W, const int* __restrict__ n_items_dev) {
+    if (n_items_dev) n_items = min(n_items, *n_items_dev);
+    __shared__ FillItem work_all[DEC_WARPS][DEC_BATCH];
+    __shared__ float grid_all[DEC_WARPS][DEC_BATCH][48];
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    FillItem* work = work_all[wid];
     const size_t row_floats = (size_t)3 * W;
     const int n_warps = gridDim.x * DEC_WARPS;
     const int gw = blockIdx.x * DEC_WARPS + wid;
-    // round r of this warp: item r * n_warps + gw (r even) or r * n_warps + n_warps - 1 - gw (r odd)
-    auto item_index = [&](int r) { return (long long)r * n_warps + ((r & 1) ? n_warps - 1 - gw : gw); };
     for (int round0 = 0; (long long)round0 * n_warps < n_items; round0 += DEC_BATCH) {
         __syncwarp();  // this warp's readers of the previous batch are done
+        bool mine = false;
+        int grid = -1;
         if (lane < DEC_BATCH) {
-            const long long idx = item_index(round0 + lane);
-            int2 itm = make_int2(-1, 0);
-            if (idx < n_items) itm = items[idx];
-            bitem[lane] = itm;
-            if (itm.x >= 0 && itm.x < n_tiles) {
-                const WeftTileDecodeDesc dd = descs[itm.x];
-                bdesc[lane] = dd;
-                if (desc_ok(dd) && dd.prim_count >= 1) bprim[lane] = load_prim(prims + dd.prim_offset);
+            const long long idx = item_index(round0 + lane, n_warps, gw);
+            int2 item = make_int2(-1, 0);
+            if (idx < n_items) item = items[idx];
+            if (item.x >= 0 && item.x < n_tiles && item.y >= 0) {
+                const WeftTileDecodeDesc d = descs[item.x];
+                if (desc_ok(d) && d.prim_count == 1) {
+                    const WeftPrim p = load_prim(prims + d.prim_offset);
+                    FillItem f;
+                    mine = fill_item(d, p.kind, res1, n_res1) && item_rect(item, d, H, W, f.r0, f.r1, f.xa, f.xb);
+                    if (mine) {
+                        grid = res1 != nullptr && n_res1 > 0 && d.res1_index >= 0 ? d.res1_index : -1;
+                        f.gy0 = d.target_y0;
+                        f.x0 = d.target_x0;
+                        f.w = d.target_w;
+                        f.grid = grid;
+                        // the blend over black and the RES0 add, once per item
+                        const Prep c = prep_prim(p);
+                        f.c0 = clamp01(blend(c.cr, c.a, 0.0f) + d.res0_r);
+                        f.c1 = clamp01(blend(c.cg, c.a, 0.0f) + d.res0_g);
+                        f.c2 = clamp01(blend(c.cb, c.a, 0.0f) + d.res0_b);
+                        f.gscale = (float)(4.0 / (double)d.target_h);  // RES1 is upsampled at the cropped tile's height
+                        work[lane] = f;
+                    }
+                }
             }
+        }
+        const unsigned todo_all = __ballot_sync(FULL, mine);
+        for (unsigned g = __ballot_sync(FULL, mine && grid >= 0); g; g &= g - 1) {
+            const int b = __ffs(g) - 1;
+            const size_t at = (size_t)__shfl_sync(FULL, grid, b) * 48;
+            grid_all[wid][b][lane] = res1[at + lane];
+            if (lane < 16) grid_all[wid][b][32 + lane] = res1[at + 32 + lane];
         }
         __syncwarp();
-        for (int b = 0; b < DEC_BATCH; ++b) {
-            if ((long long)(round0 + b) * n_warps >= n_items) break;
-            if (item_index(round0 + b) >= n_items) continue;  // this warp has no item in the round
-            const int2 item = bitem[b];
-            __syncwarp();  // this warp's readers of sp/grid/ctrl from the previous item are done
-            if (item.x < 0 || item.x >= n_tiles || item.y < 0) {
-                if (lane == 0) report(WEFTK_E_ARG);
-                continue;
+        for (unsigned todo = todo_all; todo; todo &= todo - 1) {
+            const int b = __ffs(todo) - 1;
+            const FillItem f = work[b];
+            if (f.grid >= 0) {
+                if constexpr (ALIGNED)
+                    fill_rows_res1(out, row_floats, f.gy0, f.r0, f.r1, f.x0, f.w, f.xa, f.xb, f.gscale,
+                                   grid_all[wid][b], f.c0, f.c1, f.c2, lane);
+                else
+                    fill_rows_res1_any(out, row_floats, f.gy0, f.r0, f.r1, f.x0, f.w, f.xa, f.xb, f.gscale,
+                                       grid_all[wid][b], f.c0, f.c1, f.c2, lane);
+            } else {
+                if constexpr (ALIGNED)
+                    fill_rows(out, row_floats, f.gy0, f.r0, f.r1, f.xa, f.xb, f.c0, f.c1, f.c2, lane);
+                else
+                    fill_rows_any(out, row_floats, f.gy0, f.r0, f.r1, f.xa, f.xb, f.c0, f.c1, f.c2, lane);
             }
-            render_item(item, bdesc[b], bprim[b], prims, cp48, n_cp48, res1, n_res1, out, H, W, w_aligned,
-                        row_floats, sp_all[wid], grid_all[wid], ctrl_all[wid], lane);
         }
     }
+    asm volatile("griddepcontrol.wait;" ::: "memory");  // complete only after the kernel beside it
 }
 
 int launch_score_evals(const WeftEval* d_evals, int n_evals, const WeftPrim* d_prims, const float* d_tiles,
@@ -606,10 +689,23 @@ int launch_render_tiles(const WeftTileDecodeDesc* d_descs, int n_tiles, const in
     int dev = 0, sms = 148;
     WEFTK_CUDA(cudaGetDevice(&dev));
     WEFTK_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    const int blocks = std::min((n_items + DEC_WARPS - 1) / DEC_WARPS, sms * DEC_MINB);
-    render_tiles_kernel<<<blocks, DEC_THREADS, 0, stream>>>(d_descs, n_tiles, d_items, n_items, d_prims, d_cp48,
-                                                            n_cp48, d_res1, n_res1, d_out, out_h, out_w, d_n_items);
+    const int wanted = (n_items + DEC_WARPS - 1) / DEC_WARPS;
+    render_tiles_kernel<<<std::min(n_items, sms * DEC_MINB), DEC_THREADS, 0, stream>>>(
+        d_descs, n_tiles, d_items, n_items, d_prims, d_cp48, n_cp48, d_res1, n_res1, d_out, out_h, out_w, d_n_items);
     WEFTK_CUDA(cudaGetLastError());
+    // the fills start once every CTA of the kernel above has started (so all work before it is done)
+    const bool aligned = (out_w & 3) == 0 && (reinterpret_cast<uintptr_t>(d_out) & 15) == 0;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)std::min(wanted, sms * FILL_MINB));
+    cfg.blockDim = dim3(DEC_THREADS);
+    cfg.stream = stream;
+    cudaLaunchAttribute attr = {};
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    WEFTK_CUDA(cudaLaunchKernelEx(&cfg, aligned ? render_fill_kernel<true> : render_fill_kernel<false>, d_descs, n_tiles,
+                                  d_items, n_items, d_prims, d_res1, n_res1, d_out, out_h, out_w, d_n_items));
     return WEFTK_OK;
 }
 
