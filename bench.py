@@ -1209,10 +1209,10 @@ def run_weft(args, world, rank, local, executor, cores):
     d_refine_tflops = d_flops * args.refine_steps / (dbd["refine_ms"] * 1e-3) / 1e12 if dbd["refine_ms"] else 0.0
     d_init_tflops = dbd["work"][1] / (dbd["init_score_ms"] * 1e-3) / 1e12 if dbd["init_score_ms"] else 0.0
     n_cls = sum(1 for k in (8, 16, 32) if drf.fit.n_items[k])
-    # moments, reset, prepare, begin, select, end, scoring (one per size class), refine start, one
-    # launch for all refine steps, wire-grid snap (+ the pool generation, one launch per tile side,
-    # in fit_total)
-    ref_launches = 9 + n_cls
+    # moments, reset, prepare, begin, clear, queue, constants and scoring (one each per size class),
+    # select, end, refine start, two launches for all refine steps (constant and linear layers),
+    # wire-grid snap (+ the pool generation, one launch per tile side, in fit_total)
+    ref_launches = 12 + 2 * n_cls
     # what the Adam steps add: RD of the same init round's picks without them
     init_rd = rd_of_params(dss, drf.rf.start, tiles, patches, img, args.size)
 
