@@ -1082,10 +1082,10 @@ def run_weft(args, world, rank, local, executor, cores):
     clocks = sampler.stop()
     ctl = fit.control()
     max_rounds = rate.max_rounds(QUALITY)
-    # kernels per step: reset, prepare; init round: begin, scoring per class, select, end; every
-    # greedy round (run or skipped): begin, scoring per class, select, end, control, re-seed; the
-    # selected stacks snapped to the wire grid
-    launches_per_step = 2 + (3 + n_classes) + max_rounds * (5 + n_classes) + 1
+    # kernels per step: reset, prepare, begin, clear; init round: queue, constants and scoring per
+    # class, select, end; every greedy round (run or skipped): queue, scoring per class, select, end,
+    # re-seed; the marks cleared, the selected stacks snapped to the wire grid
+    launches_per_step = 4 + (3 + 2 * n_classes) + max_rounds * (4 + n_classes) + 2
     import ctypes
 
     ms_total = ev0.elapsed_time(ev1)

@@ -159,12 +159,16 @@ __device__ __noinline__ void bicubic_pixel(const float* ctrl, int lx, int ly, in
 // tiles, 1 in 17 evaluated, into 3840 x 2160 take 38 us (99.5 MB: 15 us), and 57 with both sorts in one
 // kernel, whose 127 registers left 11 warps a SM to the fills; 1919 x 1079 with RES1 grids, whose rows
 // are not aligned, take 27 us, and 55 with four pixels a lane and 12 strided stores for each.  With four
-// layers in every tile, 3840 x 2160, 184 us, and 230 with a warp to an item; 24 layers, 1024 x 1024,
-// 141 and 144.
+// layers in every tile, 3840 x 2160, 213 us, and 230 with a warp to an item; 24 layers, 1024 x 1024,
+// 146 and 144.
 constexpr int DEC_ITEM_GROUPS = WEFTK_DECODE_ITEM_GROUPS;
 constexpr int DEC_WARPS = DEC_THREADS / 32;
 static_assert((DEC_WARPS & (DEC_WARPS - 1)) == 0, "steps are dealt out modulo DEC_WARPS");
 constexpr int DEC_MINB = 4;  // resident CTAs per SM the register budget is set for
+// CTAs per SM of the per-pixel kernel: one place less than fit, so that the fills start beside it instead of
+// after it.  A picture of lone layers, 6 % of them linear, into 3840 x 2160: 32 us at 3, 34 at 4 (30 at 2);
+// four layers in every tile: 213 at 3, 187 at 4 (255 at 2)
+constexpr int DEC_CTAS = 3;
 constexpr int DEC_BATCH = 8;
 constexpr int FILL_MINB = 8;  // the same for the fill kernel
 
@@ -690,7 +694,7 @@ int launch_render_tiles(const WeftTileDecodeDesc* d_descs, int n_tiles, const in
     WEFTK_CUDA(cudaGetDevice(&dev));
     WEFTK_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
     const int wanted = (n_items + DEC_WARPS - 1) / DEC_WARPS;
-    render_tiles_kernel<<<std::min(n_items, sms * DEC_MINB), DEC_THREADS, 0, stream>>>(
+    render_tiles_kernel<<<std::min(n_items, sms * DEC_CTAS), DEC_THREADS, 0, stream>>>(
         d_descs, n_tiles, d_items, n_items, d_prims, d_cp48, n_cp48, d_res1, n_res1, d_out, out_h, out_w, d_n_items);
     WEFTK_CUDA(cudaGetLastError());
     // the fills start once every CTA of the kernel above has started (so all work before it is done)
