@@ -34,10 +34,14 @@ extern __device__ int g_device_status;
 // Basis and zigzag tables for block sides n = 2, 4, ..., 64, back to back: side n = 2^L starts
 // at (4^L - 4) / 3.
 constexpr int kDctTab = 5460;
-__device__ double g_dct_basis[kDctTab];  // [k * n + x] = A[k][x]
-__device__ short g_dct_zigzag[kDctTab];  // [u * n + v] = zigzag scan position of (u, v)
+__device__ __align__(16) double g_dct_basis[kDctTab];  // [k * n + x] = A[k][x]; copied two at a time
+__device__ short g_dct_zigzag[kDctTab];                // [u * n + v] = zigzag scan position of (u, v)
 
 __host__ __device__ constexpr int dct_tab_off(int log2n) { return ((1 << (2 * log2n)) - 4) / 3; }
+static_assert(__alignof__(g_dct_basis) >= alignof(double2), "the basis is read as double2");
+static_assert(dct_tab_off(1) % 2 == 0 && dct_tab_off(2) % 2 == 0 && dct_tab_off(3) % 2 == 0 &&
+                  dct_tab_off(4) % 2 == 0 && dct_tab_off(5) % 2 == 0 && dct_tab_off(6) % 2 == 0,
+              "every side's basis starts on a double2");
 
 __device__ __forceinline__ int ilog2(int n) { return 31 - __clz(n); }
 
@@ -75,6 +79,9 @@ constexpr int kDctBlockWords = 4640;  // doubles of one staged block set: the la
 constexpr int kDctSteps = 252;        // steps of all block sides: side 2^L has 2^(L+1) at 2^(L+1) - 4
 __host__ __device__ constexpr int dct_pitch(int n) { return n >= 16 ? n + 2 : n; }
 __host__ __device__ constexpr int dct_slot_words(int s) { return s * dct_pitch(s) + 2; }
+static_assert(dct_pitch(2) % 2 == 0 && dct_pitch(4) % 2 == 0 && dct_pitch(8) % 2 == 0 && dct_pitch(16) % 2 == 0 &&
+                  dct_pitch(32) % 2 == 0 && dct_pitch(64) % 2 == 0 && kDctBlockWords % 2 == 0 && kDctSteps % 2 == 0,
+              "rows of a staged block, the blocks and the staged basis start on a double2");
 static_assert(256 * dct_slot_words(4) <= kDctBlockWords && 64 * dct_slot_words(8) <= kDctBlockWords &&
                   16 * dct_slot_words(16) <= kDctBlockWords && 4 * dct_slot_words(32) <= kDctBlockWords &&
                   dct_slot_words(64) <= kDctBlockWords,
@@ -158,7 +165,7 @@ __device__ __forceinline__ void dct_cols(const double* __restrict__ A, const dou
 // HALF: 4:2:0 (chroma mode 2)
 template <bool HALF>
 __global__ void __launch_bounds__(DC_THREADS, 2) dct_layer_kernel(DctLayer L) {
-    extern __shared__ double dct_smem[];
+    extern __shared__ __align__(16) double dct_smem[];
     double* X = dct_smem;                     // dequantized blocks [slot][u * pitch + v]
     double* T = X + kDctBlockWords;           // after the pass along v: [slot][u * pitch + x]
     double* steps = T + kDctBlockWords;       // luma, chroma
