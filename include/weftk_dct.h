@@ -21,6 +21,7 @@ extern "C" {
 #endif
 
 #define WEFTK_DCT_MAX_TILE 64 /* largest tile side (Y block); chroma blocks go down to 2 */
+#define WEFTK_DCT_FOLLOWS 0x100 /* added to band_layout: see weftk_dct_apply */
 
 /* One tile that carries DCT coefficients: 64 bytes.  Channel c's block is n x n with n = size,
  * or size / 2 for the Cb / Cr blocks of 4:2:0 (chroma_mode 2).  The quantized coefficient of
@@ -46,7 +47,11 @@ typedef struct WeftDctTile {
  * must not overlap (quadtree tiles never do): each pixel is written by one thread.
  *   chroma_mode  0 RGB, 1 YCbCr 4:4:4, 2 YCbCr 4:2:0 (BT.601 residual matrices; chroma step
  *                quant_step * 1.5; 4:2:0 chroma upsampled by pixel repetition)
- *   band_layout  0 tile-major, 1 band-major zigzag (see WeftDctTile)
+ *   band_layout  0 tile-major, 1 band-major zigzag (see WeftDctTile); plus WEFTK_DCT_FOLLOWS when an
+ *                earlier weftk_dct_apply without it, of at least one tile, took its tiles and coefficients
+ *                from the same arrays on this stream, and nothing writes them in between (the
+ *                further tile sides of one layer).  Such a launch may start beside the one before it; without the flag a launch
+ *                starts after all earlier work on the stream, so its inputs may come from a kernel
  *   freq_alpha   > 0: coefficient (u, v) of an n x n block uses step * (1 + alpha (u + v) / (2 (n - 1)))
  *   max_size     largest d_tiles[i].size in this launch (sizes the shared-memory staging)
  *   clip_all     != 0: afterwards clip every pixel of the image to [0, 1], as the reference's

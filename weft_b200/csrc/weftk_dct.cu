@@ -70,7 +70,7 @@ __global__ void dct_tables_kernel() {
 
 // The layer's kernel: 256 threads take 4096 pixels' worth of tiles of one side's class (one tile of 64,
 // 64 tiles of 8), so the classes of a picture are a few hundred equal CTAs, two per SM; the launches of the
-// classes overlap (a launch may start beside the one before it).  A thread owns a 4 x 4 set of a block's outputs, rows and columns n / 4 apart, so that
+// classes overlap (a launch with WEFTK_DCT_FOLLOWS may start beside the one before it).  A thread owns a 4 x 4 set of a block's outputs, rows and columns n / 4 apart, so that
 // neighbouring lanes read and write neighbouring columns; per step of a pass it reads 4 + 4 values for 16
 // float64 multiply-adds.  Cb and Cr of 4:2:0 go together, a quarter of the threads each.  Quantisation
 // steps depend on u + v only and are tabulated per CTA.
@@ -174,8 +174,10 @@ __global__ void __launch_bounds__(DC_THREADS, 2) dct_layer_kernel(DctLayer L) {
     double* basis = reinterpret_cast<double*>(R);
     constexpr int R_PLANE = HALF ? DC_PIXELS / 4 : DC_PIXELS;
     const int tid = threadIdx.x;
-    // the launch that follows may be the layer's next class: it can start beside this one, and does its
-    // transforms, but waits for this one (below) before it touches the image
+    // the launch that follows may be the layer's next class (WEFTK_DCT_FOLLOWS): it can start beside this
+    // one, and does its transforms, but waits for this one (below) before it touches the image.  Its
+    // descriptors and coefficients are complete, since the layer's first launch started after all work
+    // before it
     asm volatile("griddepcontrol.launch_dependents;");
     const int LS = L.log_side;
     const int log_slots = 12 - 2 * LS, log_tpt = 2 * LS - 4;  // slots * threads per tile = 256
@@ -693,6 +695,8 @@ extern "C" int weftk_dct_apply(const WeftDctTile* d_tiles, int n_tiles, const in
     static_assert(sizeof(WeftDctTile) == 64, "WeftDctTile must be 64 bytes");
     WEFTK_REQUIRE(n_tiles >= 0 && n_coeffs >= 0, "dct_apply: negative count");
     WEFTK_REQUIRE(chroma_mode >= 0 && chroma_mode <= 2, "dct_apply: chroma_mode must be 0, 1 or 2");
+    const bool follows = (band_layout & WEFTK_DCT_FOLLOWS) != 0;
+    band_layout &= ~WEFTK_DCT_FOLLOWS;
     WEFTK_REQUIRE(band_layout == 0 || band_layout == 1, "dct_apply: layout must be 0 or 1");
     WEFTK_REQUIRE(width > 0 && height > 0 && d_image, "dct_apply: bad image");
     WEFTK_REQUIRE(max_size >= 4 && max_size <= WEFTK_DCT_MAX_TILE && (max_size & (max_size - 1)) == 0,
@@ -718,8 +722,10 @@ extern "C" int weftk_dct_apply(const WeftDctTile* d_tiles, int n_tiles, const in
         cudaLaunchAttribute attr = {};
         attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
         attr.val.programmaticStreamSerializationAllowed = 1;
+        // without the flag an ordinary launch: it reads its inputs before griddepcontrol.wait, so whatever
+        // wrote them on the stream has to be complete when it starts
         cfg.attrs = &attr;
-        cfg.numAttrs = 1;
+        cfg.numAttrs = follows ? 1 : 0;
         WEFTK_CUDA(cudaLaunchKernelEx(&cfg, kernel, L));
     }
     if (clip_all) {

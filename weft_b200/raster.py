@@ -25,6 +25,7 @@ import numpy as np
 from . import _lib
 from ._lib import DCT_TILE_DTYPE
 
+DCT_FOLLOWS = 0x100  # WEFTK_DCT_FOLLOWS
 _HEADERS = {5: "<BBBBffHIII", 4: "<BBBBffHII", 3: "<BBffHII", 2: "<BBffHI"}
 
 
@@ -194,9 +195,10 @@ class DctLaunch:
 
     def run(self, image, stream: int, clip_all: bool = True) -> None:
         b = self.block
-        for s, lo, hi in self.groups:
+        for i, (s, lo, hi) in enumerate(self.groups):
+            layout = b.layout | (DCT_FOLLOWS if i else 0)  # the layer's further sides overlap the one before
             _lib.check(self.lib.weftk_dct_apply(_lib.ptr(self.t_descs) + lo * DCT_TILE_DTYPE.itemsize, hi - lo,
-                                                _lib.ptr(self.t_coeffs), int(b.coeffs.size), b.chroma_mode, b.layout,
+                                                _lib.ptr(self.t_coeffs), int(b.coeffs.size), b.chroma_mode, layout,
                                                 b.quant_step, b.freq_alpha, s, _lib.ptr(image), self.width,
                                                 self.height, 0, stream), "weftk_dct_apply")
         if clip_all:
