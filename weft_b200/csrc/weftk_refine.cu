@@ -838,14 +838,13 @@ __device__ __forceinline__ void general_backward(const Layers& S, int K, const R
                 al = fmaf(dLda, cov, al);
                 const float dLdcov = dLda * A;
                 float ax, ay, vx, vy, ux, uy;
-                int sg = 0;
+                float te[2] = {0.0f, 0.0f};  // a curve's segment: the parameters of its ends
                 if (line) {
                     ax = Q.q[0]; ay = Q.q[1]; vx = Q.q[2]; vy = Q.q[3]; ux = Q.q[4]; uy = Q.q[5];
                 } else {
-                    sg = h.seg[k][j];
-                    const float4 s0 = S.seg[k][sg][0];
-                    const float2 s1 = *reinterpret_cast<const float2*>(&S.seg[k][sg][1]);
-                    ax = s0.x; ay = s0.y; vx = s0.z; vy = s0.w; ux = s1.x; uy = s1.y;
+                    const int sg = h.seg[k][j];
+                    const float4 s0 = S.seg[k][sg][0], s1 = S.seg[k][sg][1];
+                    ax = s0.x; ay = s0.y; vx = s0.z; vy = s0.w; ux = s1.x; uy = s1.y; te[0] = s1.z; te[1] = s1.w;
                 }
                 const float dx = px.x[j] - ax, dy = px.y[j] - ay;
                 const float t = clamp01(fmaf(dx, ux, dy * uy));
@@ -862,12 +861,10 @@ __device__ __forceinline__ void general_backward(const Layers& S, int K, const R
                     d[2] += gex;
                     d[3] += gey;
                 } else {
-                    // polyline points are Bezier samples q_i = u^2 P0 + 2ut C + t^2 P1
+                    // polyline points are Bezier samples q_i = u^2 P0 + 2ut C + t^2 P1, at the forward pass's t
 #pragma unroll
                     for (int e2 = 0; e2 < 2; ++e2) {
-                        const int i = sg + e2;
-                        const float ti = (i >= 31) ? 1.0f : (float)i * (1.0f / 31.0f);
-                        const float ui = 1.0f - ti;
+                        const float ti = te[e2], ui = 1.0f - ti;
                         const float w0 = ui * ui, w1 = 2.0f * ui * ti, w2 = ti * ti;
                         const float gx = e2 ? gex : gsx, gy = e2 ? gey : gsy;
                         d[0] = fmaf(w0, gx, d[0]);
@@ -1130,10 +1127,11 @@ __device__ __forceinline__ void general_tile(const WeftStackSet& set, float* __r
             const float x = __fadd_rn(__fadd_rn(__fmul_rn(uu, r[0]), __fmul_rn(ut2, r[2])), __fmul_rn(t2, r[4]));
             const float y = __fadd_rn(__fadd_rn(__fmul_rn(uu, r[1]), __fmul_rn(ut2, r[3])), __fmul_rn(t2, r[5]));
             const float vx = __fsub_rn(__shfl_down_sync(FULL, x, 1), x), vy = __fsub_rn(__shfl_down_sync(FULL, y, 1), y);
+            const float next = __shfl_down_sync(FULL, tt, 1);  // the ends' parameters, for the backward pass
             const float den = __fadd_rn(__fadd_rn(__fmul_rn(vx, vx), __fmul_rn(vy, vy)), 1e-8f);
             if (lane < 31) {
                 seg[k][lane][0] = make_float4(x, y, vx, vy);
-                seg[k][lane][1] = make_float4(__fdiv_rn(vx, den), __fdiv_rn(vy, den), 0.0f, 0.0f);
+                seg[k][lane][1] = make_float4(__fdiv_rn(vx, den), __fdiv_rn(vy, den), tt, next);
             }
         }
         if (BWD)
