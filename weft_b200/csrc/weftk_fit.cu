@@ -468,10 +468,15 @@ struct ScoreSmem {
     float red[WPC > 1 ? MAX_ITEM : 1][WPC];
 };
 
-// What a thread's candidates cost (WeftFitState.work); added up once per CTA: an atomic per item on the
-// two counters serialised the CTAs of a launch.
+// What a thread's candidates cost (WeftFitState.work): those evaluated, so a curve counts once its bound
+// has let it through.  Added up once per CTA: an atomic per item on the two counters serialised the
+// CTAs of a launch.
 struct Work {
     unsigned long long px = 0, ops = 0;
+    __device__ __forceinline__ void add(int pixels, int kind) {
+        px += pixels;
+        ops += (unsigned long long)pixels * (unsigned long long)(kind_ops(kind) + 9);
+    }
 };
 
 __device__ __forceinline__ void flush_work(const WeftFitState& st, Work w) {
@@ -549,10 +554,8 @@ __device__ __forceinline__ void score_item(const WeftFitState& st, const int* __
     if (live) {
         const int pos = base + __popc(bal & ((1u << lane) - 1u));
         const Prep mine = load_prep(st, my_slot);
-        // algorithmic operations: every live candidate over the pixels the item covers
-        work.px += WPC * 32 * PPL;
-        work.ops += (unsigned long long)(WPC * 32 * PPL) * (unsigned long long)(kind_ops(mine.kind) + 9);
         my_curve = mine.kind == K_CURVE;
+        if (!my_curve) work.add(WPC * 32 * PPL, mine.kind);  // the pixels the item covers
         put_prep(s_prep[pos], mine);
         s_slot[pos] = (int)(my_slot - off);
     }
@@ -671,6 +674,7 @@ __device__ __forceinline__ void score_item(const WeftFitState& st, const int* __
         }
         float a[PPL], sr[PPL], sg[PPL], sb[PPL];
         if (P.kind == K_CURVE) {
+            if (wig == 0 && lane == 0) work.add(WPC * 32 * PPL, K_CURVE);
             put_seg2(s_seg[warp][lane], lane_segment(P, lane));
             __syncwarp();
 #pragma unroll
@@ -834,9 +838,8 @@ __device__ __forceinline__ void score_warp_item(const WeftFitState& st, const in
     if (live) {
         const int pos = __popc(bal & ((1u << lane) - 1u));
         const Prep r = load_prep(st, my_slot);
-        work.px += TS * TS;
-        work.ops += (unsigned long long)(TS * TS) * (unsigned long long)(kind_ops(r.kind) + 9);
         curve = r.kind == K_CURVE;
+        if (!curve) work.add(TS * TS, r.kind);
         put_prep(sm.prep[pos], r);
         sm.slot[pos] = (int)(my_slot - off);
     }
@@ -910,6 +913,7 @@ __device__ __forceinline__ void score_warp_item(const WeftFitState& st, const in
                     if (lane == c) mine = __int_as_float(0x7f800000);
                     continue;
                 }
+                if (lane == 0) work.add(TS * TS, K_CURVE);
                 put_seg2(sm.seg[lane], lane_segment(P, lane));
                 __syncwarp();
 #pragma unroll
