@@ -235,7 +235,7 @@ def decode_bench(fit, tiles, width, height, out_w, out_h, iters, peak, patches=N
     import torch
 
     from weft_b200 import _lib
-    from weft_b200.render import build_scene, decode_items
+    from weft_b200.render import build_scene, decode_items, walk_flags
 
     class _Rec:
         __slots__ = ("primitives", "residual_rgb")
@@ -262,6 +262,7 @@ def decode_bench(fit, tiles, width, height, out_w, out_h, iters, peak, patches=N
     t_r = torch.from_numpy(np.ascontiguousarray(res1_tab)).to(dev) if n_res1 else None
     out = torch.empty((th, tw, 3), dtype=torch.float32, device=dev)
     items = decode_items(descs, th, tw, prims)
+    flags = walk_flags(descs, prims)
     t_i = torch.from_numpy(items).to(dev)
     flush = torch.empty(64 * 1024 * 1024, dtype=torch.float32, device=dev)
     lib = _lib.lib_for_device(dev.index)
@@ -270,7 +271,7 @@ def decode_bench(fit, tiles, width, height, out_w, out_h, iters, peak, patches=N
     def launch(o=out):
         _lib.check(lib.weftk_render_tiles(_lib.ptr(t_d), len(descs), _lib.ptr(t_i), len(items), _lib.ptr(t_p),
                                           _lib.ptr(t_c), len(cp48), _lib.ptr(t_r) if n_res1 else 0, n_res1,
-                                          _lib.ptr(o), th, tw, 0,
+                                          _lib.ptr(o), th, tw, flags,
                                           stream.cuda_stream), "weftk_render_tiles")
 
     for _ in range(3):
@@ -382,7 +383,7 @@ def raster_bench(fit, tiles, patches, size, out_w, out_h, iters, peak):
 
     from weft_b200 import _lib, raster
     from weft_b200.encode import residuals_from_recon
-    from weft_b200.render import build_scene, decode_items
+    from weft_b200.render import build_scene, decode_items, walk_flags
 
     class _Rec:
         __slots__ = ("primitives", "residual_rgb")
@@ -402,6 +403,7 @@ def raster_bench(fit, tiles, patches, size, out_w, out_h, iters, peak):
     t_c = torch.from_numpy(np.ascontiguousarray(cp48)).to(dev) if len(cp48) else None
     t_r = torch.from_numpy(np.ascontiguousarray(res1_tab)).to(dev)
     items = decode_items(descs, th, tw, prims)
+    flags = walk_flags(descs, prims)
     t_i = torch.from_numpy(items).to(dev)
     img = torch.zeros((th, tw, 3), dtype=torch.float32, device=dev)
     base = torch.empty_like(img)
@@ -414,7 +416,7 @@ def raster_bench(fit, tiles, patches, size, out_w, out_h, iters, peak):
     def walk():
         _lib.check(lib.weftk_render_tiles(_lib.ptr(t_d), len(descs), _lib.ptr(t_i), len(items), _lib.ptr(t_p),
                                           _lib.ptr(t_c), len(cp48), _lib.ptr(t_r), len(res1_tab), _lib.ptr(img),
-                                          th, tw, 0, stream.cuda_stream), "weftk_render_tiles")
+                                          th, tw, flags, stream.cuda_stream), "weftk_render_tiles")
 
     def timed(fn, prep=None):
         for _ in range(3):

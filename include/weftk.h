@@ -130,15 +130,19 @@ int weftk_score_evals_host(const WeftEval* h_evals, int n_evals, const WeftPrim*
  *   d_cp48  [n_cp48 * 48]  control grids for kind-5 tiles (may be NULL)
  *   d_res1  [n_res1 * 48]  RES1 grids, (4, 4, 3) row-major, float (may be NULL;
  *                          res1_index is ignored when n_res1 == 0)
+ *   flags   0, or WEFTK_WALK_LAYERED for a picture with one evaluated layer (any but a lone
+ *         constant) for two tiles, or more: the per-pixel kernel then takes every place on
+ *         the chip at once.  The image is the same.
  * Tiles with more than 48 primitives, a rect side outside 1..8192 or an
  * out-of-range grid index are skipped and reported through weftk_device_status.
  */
 #define WEFTK_DECODE_ITEM_GROUPS 256
+#define WEFTK_WALK_LAYERED 1
 int weftk_render_tiles(const WeftTileDecodeDesc* d_descs, int n_tiles, const int32_t* d_items, int n_items,
                        const WeftPrim* d_prims, const float* d_cp48, int n_cp48, const float* d_res1, int n_res1,
                        float* d_out, int out_h, int out_w, int flags, void* stream);
 
-/* Synchronous host-buffer form of weftk_render_tiles (gpu_render_tiles_to_image). */
+/* Synchronous host-buffer form of weftk_render_tiles (gpu_render_tiles_to_image); it finds the flag itself. */
 int weftk_render_tiles_host(const WeftTileDecodeDesc* h_descs, int n_tiles, const WeftPrim* h_prims,
                             int n_prims, const float* h_cp48, int n_cp48, const float* h_res1, int n_res1,
                             float* h_out, int out_h, int out_w, int flags);

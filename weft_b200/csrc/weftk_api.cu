@@ -19,7 +19,8 @@ namespace weftk {
 
 int launch_score_evals(const WeftEval*, int, const WeftPrim*, const float*, float*, int, cudaStream_t);
 int launch_render_tiles(const WeftTileDecodeDesc*, int, const int2*, int, const WeftPrim*, const float*, int,
-                        const float*, int, float*, int, int, cudaStream_t, const int* d_n_items = nullptr);
+                        const float*, int, float*, int, int, bool layered, cudaStream_t,
+                        const int* d_n_items = nullptr);
 int read_device_status(int* status, bool clear);
 
 static thread_local std::string t_last_error;
@@ -157,9 +158,9 @@ int weftk_score_evals_host(const WeftEval* h_evals, int n_evals, const WeftPrim*
 int weftk_render_tiles(const WeftTileDecodeDesc* d_descs, int n_tiles, const int32_t* d_items, int n_items,
                        const WeftPrim* d_prims, const float* d_cp48, int n_cp48, const float* d_res1, int n_res1,
                        float* d_out, int out_h, int out_w, int flags, void* stream) {
-    (void)flags;
     return launch_render_tiles(d_descs, n_tiles, reinterpret_cast<const int2*>(d_items), n_items, d_prims, d_cp48,
-                               n_cp48, d_res1, n_res1, d_out, out_h, out_w, (cudaStream_t)stream);
+                               n_cp48, d_res1, n_res1, d_out, out_h, out_w, (flags & WEFTK_WALK_LAYERED) != 0,
+                               (cudaStream_t)stream);
 }
 
 int weftk_render_tiles_host(const WeftTileDecodeDesc* h_descs, int n_tiles, const WeftPrim* h_prims, int n_prims,
@@ -171,6 +172,7 @@ int weftk_render_tiles_host(const WeftTileDecodeDesc* h_descs, int n_tiles, cons
     // work items (tile, first row) in descending cost order (pixels, times 4 for a tile
     // evaluated per pixel: anything but a lone constant layer without a RES1 grid)
     std::vector<std::pair<long long, int2>> costed;
+    long long layers = 0;  // evaluated per pixel
     for (int i = 0; i < n_tiles; ++i) {
         const WeftTileDecodeDesc& d = h_descs[i];
         if (d.target_w > 0 && d.target_h > 0 && d.target_w <= 8192 && d.target_h <= 8192) {
@@ -190,6 +192,7 @@ int weftk_render_tiles_host(const WeftTileDecodeDesc* h_descs, int n_tiles, cons
             d.target_w <= 0 || d.target_h <= 0 || d.target_w > 8192 || d.target_h > 8192 || d.source_size <= 0 ||
             (n_res1 > 0 && d.res1_index >= n_res1))
             return fail(WEFTK_E_ARG, "render_tiles_host: tile " + std::to_string(i) + " is out of range");
+        if (d.prim_count > 1 || (d.prim_count == 1 && h_prims[d.prim_offset].kind != 0)) layers += d.prim_count;
         if (d.prim_count == 1 && h_prims[d.prim_offset].kind == 5) {
             int idx = (int)h_prims[d.prim_offset].geom[0];
             if (idx < 0 || idx >= n_cp48) return fail(WEFTK_E_ARG, "render_tiles_host: bad bicubic grid index");
@@ -222,7 +225,8 @@ int weftk_render_tiles_host(const WeftTileDecodeDesc* h_descs, int n_tiles, cons
     WEFTK_CUDA(cudaMemsetAsync(dout, 0, out_bytes, s));
     if ((rc = launch_render_tiles((const WeftTileDecodeDesc*)dd, n_tiles, (const int2*)di, (int)items.size(),
                                   (const WeftPrim*)dp, n_cp48 ? (const float*)dc : nullptr, n_cp48,
-                                  n_res1 ? (const float*)dr : nullptr, n_res1, (float*)dout, out_h, out_w, s)))
+                                  n_res1 ? (const float*)dr : nullptr, n_res1, (float*)dout, out_h, out_w,
+                                  2 * layers >= n_tiles, s)))
         return rc;
     WEFTK_CUDA(cudaMemcpyAsync(h_out, dout, out_bytes, cudaMemcpyDeviceToHost, s));
     WEFTK_CUDA(cudaStreamSynchronize(s));
@@ -264,7 +268,8 @@ int weftk_decode_scene(const WeftSceneFile* file, float* out, int on_device, int
         WEFTK_CUDA(cudaMemsetAsync(dout, 0, out_bytes, s));
         const int n_res1 = std::min(f.n_res1, f.n_tiles);
         rc = launch_render_tiles(b.descs, f.n_tiles, b.items, plan.n_items, b.prims, b.cp48, plan.cap_cp48,
-                                 n_res1 ? b.grids : nullptr, n_res1, (float*)dout, f.out_h, f.out_w, s, b.ctl + 1);
+                                 n_res1 ? b.grids : nullptr, n_res1, (float*)dout, f.out_h, f.out_w, plan.layered, s,
+                                 b.ctl + 1);
     }
     if (!rc) {
         WEFTK_CUDA(cudaMemcpyAsync(ctl, dctl, sizeof(ctl), cudaMemcpyDeviceToHost, s));

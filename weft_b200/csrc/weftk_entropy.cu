@@ -374,6 +374,8 @@ int scene_plan(const WeftSceneFile& f, ScenePlan& plan) {
     }
     if (last == 0 || last > (1u << 24)) return WEFTK_OK;  // (the slots of 16 MiB of tiles take 210 MB)
     plan.raw_len = last;
+    // a tile of one constant takes 8 bytes, an evaluated layer 9 to 21 more: about one for two tiles
+    plan.layered = plan.raw_len >= 14LL * n;
     // the chunks cover the tiles' bytes in order, without a gap
     plan.chunks.resize(f.n_chunks);
     int64_t at = 0;

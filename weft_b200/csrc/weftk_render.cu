@@ -166,9 +166,12 @@ constexpr int DEC_WARPS = DEC_THREADS / 32;
 static_assert((DEC_WARPS & (DEC_WARPS - 1)) == 0, "steps are dealt out modulo DEC_WARPS");
 constexpr int DEC_MINB = 4;  // resident CTAs per SM the register budget is set for
 // CTAs per SM of the per-pixel kernel: one place less than fit, so that the fills start beside it instead of
-// after it.  A picture of lone layers, 6 % of them linear, into 3840 x 2160: 32 us at 3, 34 at 4 (30 at 2);
-// four layers in every tile: 213 at 3, 187 at 4 (255 at 2)
-constexpr int DEC_CTAS = 3;
+// after its first look through the list, unless the picture has many layers to evaluate (`layered`).  us at
+// 3 / 4 places, 1024 x 1024 tiles into 3840 x 2160, the other tiles lone constants: 6 %, 12 %, 25 %, 50 %, all
+// of the tiles lone linear layers 31 / 34, 34 / 37, 36 / 39, 40 / 40, 53 / 48; four layers each 46 / 44,
+// 57 / 57, 85 / 79, 145 / 124, 245 / 215.  So the line lies at one evaluated layer for two tiles.
+constexpr int DEC_CTAS = 3, DEC_CTAS_LAYERED = 4;
+static_assert(DEC_CTAS_LAYERED <= DEC_MINB, "one wave");
 constexpr int DEC_BATCH = 8;
 constexpr int FILL_MINB = 8;  // the same for the fill kernel
 
@@ -684,7 +687,7 @@ int launch_score_evals(const WeftEval* d_evals, int n_evals, const WeftPrim* d_p
 
 int launch_render_tiles(const WeftTileDecodeDesc* d_descs, int n_tiles, const int2* d_items, int n_items,
                         const WeftPrim* d_prims, const float* d_cp48, int n_cp48, const float* d_res1, int n_res1,
-                        float* d_out, int out_h, int out_w, cudaStream_t stream, const int* d_n_items) {
+                        float* d_out, int out_h, int out_w, bool layered, cudaStream_t stream, const int* d_n_items) {
     if (n_tiles == 0) return WEFTK_OK;
     WEFTK_REQUIRE(n_tiles > 0 && d_descs && d_out && out_h > 0 && out_w > 0, "render_tiles: bad arguments");
     WEFTK_REQUIRE(n_cp48 >= 0 && n_res1 >= 0, "render_tiles: negative table size");
@@ -694,7 +697,7 @@ int launch_render_tiles(const WeftTileDecodeDesc* d_descs, int n_tiles, const in
     WEFTK_CUDA(cudaGetDevice(&dev));
     WEFTK_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
     const int wanted = (n_items + DEC_WARPS - 1) / DEC_WARPS;
-    render_tiles_kernel<<<std::min(n_items, sms * DEC_CTAS), DEC_THREADS, 0, stream>>>(
+    render_tiles_kernel<<<std::min(n_items, sms * (layered ? DEC_CTAS_LAYERED : DEC_CTAS)), DEC_THREADS, 0, stream>>>(
         d_descs, n_tiles, d_items, n_items, d_prims, d_cp48, n_cp48, d_res1, n_res1, d_out, out_h, out_w, d_n_items);
     WEFTK_CUDA(cudaGetLastError());
     // the fills start once every CTA of the kernel above has started (so all work before it is done)

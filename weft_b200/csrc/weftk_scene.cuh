@@ -12,6 +12,7 @@ namespace weftk {
 
 struct ScenePlan {
     bool ok;      // false: a form the general decoder handles (or refuses)
+    bool layered;  // many layers to evaluate (WEFTK_WALK_LAYERED)
     int scaled, n_items, cap_prims, cap_cp48;
     int64_t raw_len;
     double sx, sy;

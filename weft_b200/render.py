@@ -23,6 +23,7 @@ from ._lib import PRIM_DTYPE, TILE_DECODE_DTYPE
 MAX_TILE_PRIMS = 48
 DECODE_ITEM_GROUPS = 256   # WEFTK_DECODE_ITEM_GROUPS
 ITEM_PIXEL_WORK = 4        # cost of a pixel evaluated per pixel, in pixels of a constant fill
+WALK_LAYERED = 1           # WEFTK_WALK_LAYERED
 
 
 def decode_items(descs: np.ndarray, out_h: int, out_w: int, prims: np.ndarray | None = None) -> np.ndarray:
@@ -55,6 +56,17 @@ def decode_items(descs: np.ndarray, out_h: int, out_w: int, prims: np.ndarray | 
     cost = n_rows * np.repeat(w, per) * np.where(np.repeat(per_pixel, per), ITEM_PIXEL_WORK, 1)
     order = np.argsort(-cost, kind="stable")
     return np.stack([tile[order], first[order]], axis=1).astype(np.int32)
+
+
+def walk_flags(descs: np.ndarray, prims: np.ndarray) -> int:
+    """``flags`` of weftk_render_tiles for a scene: WALK_LAYERED from one evaluated layer (any but a lone
+    constant) for two tiles on."""
+    counts = descs["prim_count"].astype(np.int64)
+    if not len(prims):
+        return 0
+    first = prims["kind"][np.clip(descs["prim_offset"], 0, len(prims) - 1)]
+    layers = int(counts[(counts > 1) | ((counts == 1) & (first != 0))].sum())
+    return WALK_LAYERED if 2 * layers >= len(descs) else 0
 
 
 def pack_records(stacks) -> tuple[np.ndarray, np.ndarray, np.ndarray, np.ndarray]:
@@ -179,7 +191,8 @@ def render_scene_device(records, quad_tiles, width: int, height: int, residual_m
     t_r = torch.from_numpy(np.ascontiguousarray(res1, np.float32)).to(dev) if n_res1 else None
     lib = _lib.lib_for_device(device)
     _lib.check(lib.weftk_render_tiles(_lib.ptr(t_d), len(descs), _lib.ptr(t_i), len(items), _lib.ptr(t_p),
-                                      _lib.ptr(t_c), len(cp48), _lib.ptr(t_r), n_res1, _lib.ptr(out), th, tw, 0,
+                                      _lib.ptr(t_c), len(cp48), _lib.ptr(t_r), n_res1, _lib.ptr(out), th, tw,
+                                      walk_flags(descs, prims),
                                       torch.cuda.current_stream(dev).cuda_stream), "weftk_render_tiles")
     return out
 
