@@ -764,15 +764,17 @@ __global__ void __launch_bounds__(128, MINB) fit_score_queue_kernel(WeftFitState
         int next = 0;
         if (threadIdx.x == 0) next = atomicAdd(q_next, 1);
         WeftFitItem w = items[q_items[i / parts]];
-        const int each = (w.count + parts - 1) / parts, from = (i % parts) * each;
-        w.first += from;
-        w.count = min(each, w.count - from);
-        if (w.count <= 0) {  // (a malformed count is rejected as before)
-            if (i % parts == 0) score_item<PPL, WPC, false>(st, perm, w, expect_min, expect_max, lam, sm, work);
-        } else if (mode_init) {
-            score_item<PPL, WPC, true>(st, perm, w, expect_min, expect_max, lam, sm, work);
-        } else {
-            score_item<PPL, WPC, false>(st, perm, w, expect_min, expect_max, lam, sm, work);
+        // a malformed count is not dealt in parts, which could pass where the whole is refused: the first pull
+        // hands it on as it is
+        const bool whole = w.count <= 0 || w.count > MAX_ITEM;
+        if (!whole) {
+            const int each = (w.count + parts - 1) / parts, from = (i % parts) * each;
+            w.first += from;
+            w.count = min(each, w.count - from);
+        }
+        if (whole ? i % parts == 0 : w.count > 0) {
+            if (mode_init) score_item<PPL, WPC, true>(st, perm, w, expect_min, expect_max, lam, sm, work);
+            else score_item<PPL, WPC, false>(st, perm, w, expect_min, expect_max, lam, sm, work);
         }
         __syncthreads();  // every thread has read s_i and the item's shared buffers are free
         if (threadIdx.x == 0) s_i = next;
