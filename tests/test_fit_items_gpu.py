@@ -47,3 +47,12 @@ def _round_with(side, variant, queue, mode, item):
 def test_more_candidates_than_an_item_holds(side, variant, queue, mode, count):
     assert _round_with(side, variant, queue, mode, (0, 0, 0, 128)) == 0
     assert _round_with(side, variant, queue, mode, (0, 0, 0, count)) == -1
+
+
+@pytest.mark.parametrize("mode", [0, 1])
+@pytest.mark.parametrize("queue", [True, False])
+@pytest.mark.parametrize("side,variant", [(8, 0), (8, 2), (16, 0), (16, 1), (32, 0), (64, 1)])
+@pytest.mark.parametrize("block", [-1, -4, 4, 1 << 22, (1 << 31) - 1, -(1 << 31)])
+def test_blocks_outside_the_tile(side, variant, queue, mode, block):
+    """(1 << 22 blocks of 1024 pixels: a product past 32 bits.)"""
+    assert _round_with(side, variant, queue, mode, (0, block, 0, 64)) == -1

@@ -516,8 +516,8 @@ __device__ __forceinline__ void score_item(const WeftFitState& st, const int* __
     const bool closed_form = INIT && st.moments != nullptr;
     // a slot range outside the state's slot arrays (a malformed caller-built pool table) is
     // rejected, never scored: the per-candidate scratch is indexed by slot
-    if (ts < expect_min || ts > expect_max || w.count > MAX_ITEM || w.block * 1024 >= ts * ts || w.first < 0 ||
-        w.first + w.count > st.pool_cap[t] || st.pool_off[t] < 0 ||
+    if (ts < expect_min || ts > expect_max || w.count > MAX_ITEM || w.block < 0 || w.block >= (ts * ts + 1023) / 1024 ||
+        w.first < 0 || w.first + w.count > st.pool_cap[t] || st.pool_off[t] < 0 ||
         (long long)st.pool_off[t] + w.first + w.count > st.n_slots) {
         if (threadIdx.x == 0) fit_report(WEFTK_E_ARG);
         return;
