@@ -66,6 +66,22 @@ static int arena_get(int slot, size_t bytes, void** out, Arena& a) {
     return WEFTK_OK;
 }
 
+// Gives the buffers of a file's decode back when together they are larger than `most`; the work on them must
+// be done.
+constexpr int SCENE_SLOTS[] = {4, 5, 6, 7, 9, 10, 11, 12};
+static void arena_trim_scene(size_t most, Arena& a) {
+    size_t total = 0;
+    for (int slot : SCENE_SLOTS)
+        if (slot < (int)a.cap.size()) total += a.cap[slot];
+    if (total <= most) return;
+    for (int slot : SCENE_SLOTS) {
+        if (slot >= (int)a.ptr.size() || !a.ptr[slot]) continue;
+        cudaFree(a.ptr[slot]);
+        a.ptr[slot] = nullptr;
+        a.cap[slot] = 0;
+    }
+}
+
 static int arena_for_current(Arena** out) {
     int dev = 0;
     WEFTK_CUDA(cudaGetDevice(&dev));
@@ -233,6 +249,10 @@ int weftk_render_tiles_host(const WeftTileDecodeDesc* h_descs, int n_tiles, cons
     return check_status_after_sync();
 }
 
+// Device memory kept between files: an 8192 x 8192 picture's 5 MB of tiles need about 95 MB.  Allocating anew
+// for a larger one costs about a millisecond of the 70 and more that its pixels' copy takes.
+static constexpr size_t SCENE_KEEP = (size_t)128 << 20;
+
 int weftk_decode_scene(const WeftSceneFile* file, float* out, int on_device, int* irregular, void* stream) {
     WEFTK_REQUIRE(file && file->blob && out && irregular, "decode_scene: null pointer");
     *irregular = 1;
@@ -245,16 +265,18 @@ int weftk_decode_scene(const WeftSceneFile* file, float* out, int on_device, int
     if ((rc = arena_for_current(&a))) return rc;
     const size_t out_bytes = sizeof(float) * 3 * (size_t)f.out_h * (size_t)f.out_w;
     void *dblob, *dchunks, *draw, *dd, *dp, *dc, *dr, *di, *dctl, *dout = out;
-    if ((rc = arena_get(10, (size_t)f.blob_len, &dblob, *a))) return rc;
-    if ((rc = arena_get(11, sizeof(WeftRansChunk) * plan.chunks.size(), &dchunks, *a))) return rc;
-    if ((rc = arena_get(12, (size_t)plan.raw_len, &draw, *a))) return rc;
-    if ((rc = arena_get(13, 2 * sizeof(int), &dctl, *a))) return rc;
-    if ((rc = arena_get(4, sizeof(WeftTileDecodeDesc) * (size_t)f.n_tiles, &dd, *a))) return rc;
-    if ((rc = arena_get(5, sizeof(WeftPrim) * (size_t)plan.cap_prims, &dp, *a))) return rc;
-    if ((rc = arena_get(6, sizeof(float) * 48 * (size_t)plan.cap_cp48, &dc, *a))) return rc;
-    if ((rc = arena_get(7, sizeof(float) * 48 * (size_t)std::max(1, f.n_res1), &dr, *a))) return rc;
-    if ((rc = arena_get(9, sizeof(int2) * (size_t)std::max(1, plan.n_items), &di, *a))) return rc;
-    if (!on_device && (rc = arena_get(8, out_bytes, &dout, *a))) return rc;
+    if ((rc = arena_get(10, (size_t)f.blob_len, &dblob, *a)) ||
+        (rc = arena_get(11, sizeof(WeftRansChunk) * plan.chunks.size(), &dchunks, *a)) ||
+        (rc = arena_get(12, (size_t)plan.raw_len, &draw, *a)) || (rc = arena_get(13, 2 * sizeof(int), &dctl, *a)) ||
+        (rc = arena_get(4, sizeof(WeftTileDecodeDesc) * (size_t)f.n_tiles, &dd, *a)) ||
+        (rc = arena_get(5, sizeof(WeftPrim) * (size_t)plan.cap_prims, &dp, *a)) ||
+        (rc = arena_get(6, sizeof(float) * 48 * (size_t)plan.cap_cp48, &dc, *a)) ||
+        (rc = arena_get(7, sizeof(float) * 48 * (size_t)std::max(1, f.n_res1), &dr, *a)) ||
+        (rc = arena_get(9, sizeof(int2) * (size_t)std::max(1, plan.n_items), &di, *a)) ||
+        (!on_device && (rc = arena_get(8, out_bytes, &dout, *a)))) {
+        arena_trim_scene(SCENE_KEEP, *a);
+        return rc;
+    }
     cudaStream_t s = on_device ? (cudaStream_t)stream : a->stream;
     const SceneBuffers b = {(const uint8_t*)dblob,    (const WeftRansChunk*)dchunks, (uint8_t*)draw,
                             (WeftTileDecodeDesc*)dd,  (WeftPrim*)dp,                 (float*)dc,
@@ -277,6 +299,7 @@ int weftk_decode_scene(const WeftSceneFile* file, float* out, int on_device, int
     }
     // (the arena's buffers and the chunk list are this call's until its work is done)
     const cudaError_t e = cudaStreamSynchronize(s);
+    arena_trim_scene(SCENE_KEEP, *a);
     if (rc) return rc;
     WEFTK_CUDA(e);
     *irregular = ctl[0] != 0;
