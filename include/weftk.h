@@ -124,9 +124,9 @@ int weftk_score_evals_host(const WeftEval* h_evals, int n_evals, const WeftPrim*
  *                     ... for the rows r0 <= r < r1 of its rect that lie inside the
  *                     image (r0 = max(0, -y0), r1 = min(h, out_h - y0)).  Rows of an
  *                     item outside the image are skipped.  Any order renders the same
- *                     image; in descending order of cost (pixels, times 4 for a tile
- *                     evaluated per pixel, i.e. anything but a lone constant layer
- *                     without a RES1 grid) the warps finish together.
+ *                     image; in descending order of cost (pixels, times 4 for any tile
+ *                     but a lone constant layer without a RES1 grid) the warps finish
+ *                     together.
  *   d_cp48  [n_cp48 * 48]  control grids for kind-5 tiles (may be NULL)
  *   d_res1  [n_res1 * 48]  RES1 grids, (4, 4, 3) row-major, float (may be NULL;
  *                          res1_index is ignored when n_res1 == 0)

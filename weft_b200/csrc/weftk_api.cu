@@ -185,8 +185,8 @@ int weftk_render_tiles_host(const WeftTileDecodeDesc* h_descs, int n_tiles, cons
     (void)flags;
     WEFTK_REQUIRE(n_tiles >= 0 && out_h > 0 && out_w > 0 && h_out && n_prims >= 0 && n_cp48 >= 0 && n_res1 >= 0,
                   "render_tiles_host: bad arguments");
-    // work items (tile, first row) in descending cost order (pixels, times 4 for a tile
-    // evaluated per pixel: anything but a lone constant layer without a RES1 grid)
+    // work items (tile, first row) in descending cost order (pixels, times 4 for any tile but a
+    // lone constant layer without a RES1 grid)
     std::vector<std::pair<long long, int2>> costed;
     long long layers = 0;  // evaluated per pixel
     for (int i = 0; i < n_tiles; ++i) {

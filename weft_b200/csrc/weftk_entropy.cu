@@ -120,7 +120,7 @@ __global__ void __launch_bounds__(32) rans_decode_kernel(const uint8_t* __restri
     }
     st.word = reinterpret_cast<const unsigned*>(end);
     st.ahead = end > em ? *--st.word : 0;
-    auto refill = [&] {  // to 40 bits at least, as long as there are any
+    auto refill = [&] {  // to 32 bits at least, as long as there are any: two symbols take 16 each at most
         if (st.have <= 32) {
             st.win |= (unsigned long long)st.ahead << (32 - st.have);
             st.have += 32;

@@ -343,8 +343,8 @@ __device__ __forceinline__ void put_seg2(Seg2& d, const Seg& s) {
     d.uy = pack2(s.uy, s.uy);
 }
 
-// Alpha of a curve at PPL pixels (seg_d2 over the 31 segments, as curve_alpha_smem); an odd last
-// pixel is paired with itself.
+// Alpha of a curve at PPL pixels (seg_d2 over the 31 segments, in their order); an odd last pixel is
+// paired with itself.
 template <int PPL>
 __device__ __forceinline__ void curve_alpha2(const Prep& P, const Seg2* seg, const float (&fx)[PPL],
                                              const float (&fy)[PPL], float (&a)[PPL]) {
@@ -582,15 +582,7 @@ __device__ __forceinline__ void score_item(const WeftFitState& st, const int* __
             }
             for (int c0 = warp * 2; c0 < m; c0 += 8) {
                 const int c = min(c0 + half, m - 1);
-                Prep P;
-                {
-                    const float4 a = s_prep[c][0], b = s_prep[c][1], cc = s_prep[c][2], d = s_prep[c][3];
-                    P.kind = __float_as_int(a.x);
-                    P.a = a.y; P.cr = a.z; P.cg = a.w; P.cb = b.x;
-                    P.q[0] = b.y; P.q[1] = b.z; P.q[2] = b.w;
-                    P.q[3] = cc.x; P.q[4] = cc.y; P.q[5] = cc.z; P.q[6] = cc.w;
-                    P.q[7] = d.x; P.q[8] = d.y; P.q[9] = d.z; P.q[10] = d.w;
-                }
+                const Prep P = smem_prep(s_prep[c]);
                 float a[4], sr[4], sg[4], sb[4];
                 prim_eval<4>(P, hx, hy, a, sr, sg, sb, lane);  // no curve: no shuffles inside
                 float e = 0.0f;
@@ -663,15 +655,7 @@ __device__ __forceinline__ void score_item(const WeftFitState& st, const int* __
             }
             continue;
         }
-        Prep P;
-        {
-            const float4 a = s_prep[c][0], b = s_prep[c][1], cc = s_prep[c][2], d = s_prep[c][3];
-            P.kind = __float_as_int(a.x);
-            P.a = a.y; P.cr = a.z; P.cg = a.w; P.cb = b.x;
-            P.q[0] = b.y; P.q[1] = b.z; P.q[2] = b.w;
-            P.q[3] = cc.x; P.q[4] = cc.y; P.q[5] = cc.z; P.q[6] = cc.w;
-            P.q[7] = d.x; P.q[8] = d.y; P.q[9] = d.z; P.q[10] = d.w;
-        }
+        const Prep P = smem_prep(s_prep[c]);
         float a[PPL], sr[PPL], sg[PPL], sb[PPL];
         if (P.kind == K_CURVE) {
             if (wig == 0 && lane == 0) work.add(WPC * 32 * PPL, K_CURVE);

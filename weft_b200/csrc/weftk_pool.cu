@@ -778,10 +778,7 @@ __global__ void __launch_bounds__(NT, 1024 / NT) gen_pool_kernel(WeftPoolTables 
 
     // 6. palettes: the 13 colours (tile mean, then regions 21..32 in order), their pairwise
     //    near tests in parallel, then one thread keeps each colour that is not near one kept
-    //    before it; then the candidate list's segment sizes: the list is (edge pool) palette x 4
-    //    alphas, quadrants x 2, orientations x 5, (template pool) palette x 4, quadrants x 2,
-    //    blocks, splits x 3 or x 1, so candidate i is a function of i that any thread can
-    //    evaluate (cand_at below)
+    //    before it
     if (tid < NCOL) {
         float m[3];
         const int r = 20 + tid;

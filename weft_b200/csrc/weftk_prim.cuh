@@ -240,26 +240,6 @@ __device__ __forceinline__ void prim_eval(const Prep& P, const float (&fx)[PPL],
     }
 }
 
-// Same as prim_eval for kind K_CURVE, with the warp's 31 segments already in shared
-// memory (seg[k] = {ax, ay, vx, vy}, {ux, uy, -, -}); reads are warp-uniform broadcasts.
-template <int PPL>
-__device__ __forceinline__ void curve_alpha_smem(const Prep& P, const float4 (*seg)[2], const float (&fx)[PPL],
-                                                 const float (&fy)[PPL], float (&a)[PPL]) {
-    float best[PPL];
-#pragma unroll
-    for (int j = 0; j < PPL; ++j) best[j] = 1e18f;
-#pragma unroll 2
-    for (int k = 0; k < 31; ++k) {
-        const float4 s0 = seg[k][0];
-        const float4 s1 = seg[k][1];
-#pragma unroll
-        for (int j = 0; j < PPL; ++j)
-            best[j] = fminf(best[j], seg_d2(fx[j], fy[j], s0.x, s0.y, s0.z, s0.w, s1.x, s1.y));
-    }
-#pragma unroll
-    for (int j = 0; j < PPL; ++j) a[j] = expf(best[j] * P.q[0]) * P.a;
-}
-
 // "over" blend, identical sequence in every kernel so incremental and full renders agree bit for bit.
 __device__ __forceinline__ float blend(float s, float a, float c) {
     return __fmaf_rn(s, a, __fmul_rn(c, __fsub_rn(1.0f, a)));

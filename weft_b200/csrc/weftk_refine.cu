@@ -146,16 +146,10 @@ __device__ __forceinline__ int pick(const int (&a)[RF_CLASSES], int c) {
     return c == 0 ? a[0] : c == 1 ? a[1] : c == 2 ? a[2] : a[3];
 }
 
-// Gradient columns a layer of this kind can produce (bit i = column i).
+// Gradient columns a constant or linear layer can produce (bit i = column i).
 __device__ __forceinline__ unsigned grad_columns(int kind) {
-    switch (kind) {
-        case K_CONST: return 0x2380u;   // 7 8 9 13
-        case K_LINEAR: return 0x3f8fu;  // 0-3 7-13
-        case K_LINE: return 0x239fu;    // 0-4 7 8 9 13
-        case K_CURVE: return 0x23ffu;   // 0-6 7 8 9 13
-        case K_TRI: return 0x23bfu;     // 0-5 7 8 9 13
-        default: return 0u;
-    }
+    // 7 8 9 13; 0-3 7-13
+    return kind == K_CONST ? 0x2380u : kind == K_LINEAR ? 0x3f8fu : 0u;
 }
 
 // Bilinear node pair (lo, hi) and weight of the decoder's 4x4 residual grid for a
@@ -218,7 +212,7 @@ __device__ __forceinline__ ClEval eval_cl(const Prep& P, float px, float py) {
 }
 
 // Gradient of that layer over black (c_{-1} = 0), accumulated into acc[14]; the same chain
-// rule as layer_grad's constant and linear cases.
+// rule as general_backward's constant and linear cases.
 __device__ __forceinline__ void grad_cl(const Prep& P, const float* r, const ClEval& v, float px, float py,
                                         const float (&g)[3], float (&acc)[14]) {
     if (P.kind != K_CONST && P.kind != K_LINEAR) return;
@@ -1228,7 +1222,7 @@ __device__ __forceinline__ void general_tile(const WeftStackSet& set, float* __r
                     }
                 }
                 if (BWD && Q >= P) {
-                    const int span = Q / P;  // <= 16 lanes
+                    const int span = Q / P;  // <= 32 lanes (a 64-px tile's quadrants of 64 pixels)
                     for (int o = 1; o < span; o <<= 1)
 #pragma unroll
                         for (int u = 0; u < 12; ++u) acc[u] += __shfl_xor_sync(FULL, acc[u], o);

@@ -5,7 +5,7 @@
 // composites the whole stack for them in registers; the per-lane squared error of a
 // chunk is summed in float32 and accumulated in float64; one warp reduction per eval.
 //
-// Decode walk: work items of tile rows, one warp per item.  Two kernels run side by side: one
+// Decode walk: work items of tile rows.  Two kernels run side by side: one
 // for lone constant tiles (almost every tile of a fit at q75), which are written as runs of
 // their rows, and one for all others, per 4-pixel group with the stack composited in
 // registers.  Output is float32 HWC.
@@ -131,25 +131,23 @@ __device__ __noinline__ void bicubic_pixel(const float* ctrl, int lx, int ly, in
 // Work items: (tile, first row).  An item covers rows [first, first + R) of the tile's
 // target rect, R = max(1, WEFTK_DECODE_ITEM_GROUPS / G), where G is the number of
 // 4-pixel groups (aligned to output x multiples of 4) a rect row touches; rows outside
-// the image are skipped.  Each item is rendered by ONE warp: the warp stages its tile's
-// primitives in its own slice of shared memory and never waits on the rest of the CTA,
-// so every resident warp works on a different item.  A persistent grid of one wave
-// (every CTA resident) walks the list in rounds: in round r warp w takes item
-// r * n_warps + w when r is even and r * n_warps + n_warps - 1 - w when r is odd, so
-// with the items in descending cost order every warp gets a similar share of the work
-// (the warps' finishing times, not their item counts, set the kernel's duration).  A
-// warp fetches the records of its next DEC_BATCH items at once (item, descriptor and
-// first primitive, one item per lane), so the dependent-load chain item -> descriptor
-// -> primitive is paid once per batch instead of once per item.
+// the image are skipped.  Both kernels are persistent grids that walk the list in rounds: in
+// round r the taker w of n (a warp of the fills, a CTA of the per-pixel kernel) has item r * n + w
+// when r is even and r * n + n - 1 - w when r is odd, so with the items in descending cost order
+// every taker gets a similar share of the work (the takers' finishing times, not their item
+// counts, set the kernel's duration).  It fetches the records of several rounds at once (item,
+// descriptor and first primitive, one item per lane or thread), so the dependent-load chain
+// item -> descriptor -> primitive is paid once per batch instead of once per item.
 //
 // Two kernels walk the same list.  Both take the whole list's records, so that neither
 // needs a second list; each leaves the other's items.
-//  * render_fill_kernel: lone constant layers, with or without a RES1 grid, at 64 registers.
-//    What an item needs (clipped rect, final colour, grid) is worked out by one lane per item
-//    of the batch, and the stores are runs of the rows: where rows are 16-byte aligned, whole
-//    16-byte slots (slot s holds channels s, s+1, s+2, s mod 3 of the colour), the at most
-//    three floats at each end of a row that share a slot with the neighbouring tile one by
-//    one; else one float per lane.  Either way a warp's stores are contiguous.
+//  * render_fill_kernel: lone constant layers, with or without a RES1 grid, at 64 registers.  A
+//    warp has its items to itself and never waits on the rest of its CTA.  What an item needs
+//    (clipped rect, final colour, grid) is worked out by one lane per item of the batch, and the
+//    stores are runs of the rows: where rows are 16-byte aligned, whole 16-byte slots (slot s
+//    holds channels s, s+1, s+2, s mod 3 of the colour), the at most three floats at each end of
+//    a row that share a slot with the neighbouring tile one by one; else one float per lane.
+//    Either way a warp's stores are contiguous.
 //  * render_tiles_kernel: anything else, per 4-pixel group, at twice the registers.  A CTA
 //    looks through 128 items at once and its four warps share those that are its own, 32 groups in
 //    turn: one warp on a whole item of four layers needs 40 us, whatever the others do.
@@ -158,9 +156,9 @@ __device__ __noinline__ void bicubic_pixel(const float* ctrl, int lx, int ly, in
 // Bound: the stores' bandwidth where few tiles are evaluated per pixel.  1024 x 1024 fitted
 // tiles, 1 in 17 evaluated, into 3840 x 2160 take 38 us (99.5 MB: 15 us), and 57 with both sorts in one
 // kernel, whose 127 registers left 11 warps a SM to the fills; 1919 x 1079 with RES1 grids, whose rows
-// are not aligned, take 27 us, and 55 with four pixels a lane and 12 strided stores for each.  With four
-// layers in every tile, 3840 x 2160, 213 us, and 230 with a warp to an item; 24 layers, 1024 x 1024,
-// 146 and 144.
+// are not aligned, take 27 us, and 55 with four pixels a lane and 12 strided stores for each.  Evaluation
+// where there is much of it: 64 x 64 tiles of four layers, 3840 x 2160, 184 us, and 230 with a warp to an
+// item; of 24 layers, 1024 x 1024, 141 and 144.
 constexpr int DEC_ITEM_GROUPS = WEFTK_DECODE_ITEM_GROUPS;
 constexpr int DEC_WARPS = DEC_THREADS / 32;
 static_assert((DEC_WARPS & (DEC_WARPS - 1)) == 0, "steps are dealt out modulo DEC_WARPS");
@@ -392,7 +390,7 @@ __device__ __forceinline__ bool fill_item(const WeftTileDecodeDesc& d, int kind0
            !(res1 != nullptr && n_res1 > 0 && d.res1_index >= n_res1);
 }
 
-// One work item (tile rows) rendered by one warp; p0 is the tile's first primitive (unset
+// A warp's share of one work item (tile rows); p0 is the tile's first primitive (unset
 // when the tile has none), prepared, and geo its sampling step and RES1 scale; sp / grid / ctrl are the
 // warp's shared-memory slices.  The warp
 // takes steps part, part + DEC_WARPS, .. of the item, 32 groups each; returns how many steps it has.

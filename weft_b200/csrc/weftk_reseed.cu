@@ -43,7 +43,7 @@ constexpr int NV = 36;  // reduced values of the main pass
 struct RsShared {
     double red[RS_WARPS][NV];
     double res[NV];
-    int colcnt[64], colminy[64], colmaxy[64], rowcnt[64], rowminx[64];
+    int colcnt[64], colminy[64], colmaxy[64], rowcnt[64];
     WeftPrim cand[RS_MAX_CANDS];
     int key[RS_MAX_CANDS][KEY_LEN];
     unsigned hash[RS_MAX_CANDS];
@@ -191,7 +191,6 @@ __global__ void __launch_bounds__(RS_THREADS) fit_reseed_kernel(WeftFitState st,
         s.rowcnt[tid] = 0;
         s.colminy[tid] = INT_MAX;
         s.colmaxy[tid] = -1;
-        s.rowminx[tid] = INT_MAX;
     }
     __syncthreads();
     // numpy percentile of a float32 array, linear method, all in float32:
@@ -242,7 +241,6 @@ __global__ void __launch_bounds__(RS_THREADS) fit_reseed_kernel(WeftFitState st,
             atomicMin(&s.colminy[x], y);
             atomicMax(&s.colmaxy[x], y);
             atomicAdd(&s.rowcnt[y], 1);
-            atomicMin(&s.rowminx[y], x);
         }
     }
     block_sum(v, s);

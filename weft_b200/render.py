@@ -22,7 +22,7 @@ from ._lib import PRIM_DTYPE, TILE_DECODE_DTYPE
 
 MAX_TILE_PRIMS = 48
 DECODE_ITEM_GROUPS = 256   # WEFTK_DECODE_ITEM_GROUPS
-ITEM_PIXEL_WORK = 4        # cost of a pixel evaluated per pixel, in pixels of a constant fill
+ITEM_PIXEL_WORK = 4        # cost of a pixel that is evaluated or interpolated, in pixels of a constant fill
 WALK_LAYERED = 1           # WEFTK_WALK_LAYERED
 
 
@@ -31,9 +31,10 @@ def decode_items(descs: np.ndarray, out_h: int, out_w: int, prims: np.ndarray | 
 
     A rect row touches G 4-pixel groups aligned to output x multiples of 4; an item covers
     max(1, DECODE_ITEM_GROUPS // G) rows of its tile.  Only the rows inside the out_h x out_w
-    image get items.  The cost of an item is its pixel count, times ITEM_PIXEL_WORK for a tile
-    that is evaluated per pixel (anything but a lone constant layer without a RES1 grid; with
-    ``prims`` None every tile without a RES1 grid counts as a lone constant layer).
+    image get items.  The cost of an item is its pixel count, times ITEM_PIXEL_WORK for any tile
+    but a lone constant layer without a RES1 grid: those evaluated per pixel, and the fills that
+    interpolate a grid (with ``prims`` None every tile without a RES1 grid counts as a lone
+    constant layer).
     """
     x0 = descs["target_x0"].astype(np.int64)
     y0 = descs["target_y0"].astype(np.int64)
