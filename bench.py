@@ -211,10 +211,11 @@ class ClockSampler:
 B2B_LAUNCHES, B2B_BUFFERS = 9, 3
 INIT_SAMPLES = 5
 
-# DRAM bytes (read + write) of one init round's three scoring launches and of one refine launch
-# pair (constant + tiles kernels), 1024^2 workload, from one ncu capture of the eager pipeline
-INIT_ROUND_TRAFFIC = 82_512_384 + 2_255_104
-REFINE_TRAFFIC = 1_919_232 + 930_048
+# DRAM bytes (read + write) of one init round's launches (constants, queue and scoring of the three
+# size classes) and of one refine launch pair (constant + tiles kernels), 1024^2 workload, from one
+# ncu capture of the eager pipeline
+INIT_ROUND_TRAFFIC = 45_556_224 + 156_672
+REFINE_TRAFFIC = 1_919_488 + 909_056
 TRAFFIC_SOURCE = ("ncu dram__bytes_read.sum + dram__bytes_write.sum, summed over the kernel's launches "
                   "(python bench.py --profile-refined --steps 1 --warmup 1)")
 
@@ -1276,7 +1277,8 @@ def run_weft(args, world, rank, local, executor, cores):
         decode["cpu_baseline"] = dec_cpu
     score_roof = {"bound": "fp32", "achieved": achieved_tflops, "peak": peak_tflops, "unit": "TFLOP/s",
                   "frac": achieved_tflops / peak_tflops if peak_tflops else None, "traffic": None,
-                  "kernel": "fit_score_queue_kernel (3 tile-size classes, all rounds), plain fit",
+                  "kernel": "fit_const_*, fit_queue, fit_score_warp / fit_score_queue kernels (3 tile-size classes, all "
+                            "rounds), plain fit",
                   "peak_source": "measured FMA-loop probe on this GPU (weftk_measure_fp32_peak)",
                   "score_ms_per_step": score_ms.value / args.steps, "score_launches": n_score.value,
                   "candidate_pixels_per_step": cand_px // args.steps}
@@ -1290,7 +1292,8 @@ def run_weft(args, world, rank, local, executor, cores):
     init_roof = {"bound": "fp32", "achieved": d_init_tflops, "peak": peak_tflops, "unit": "TFLOP/s",
                  "frac": d_init_tflops / peak_tflops if peak_tflops else None, "traffic": INIT_ROUND_TRAFFIC,
                  "traffic_source": TRAFFIC_SOURCE,
-                 "kernel": "fit_score_queue_kernel, init round of the refined fit (three tile-size classes)", "ms": dbd["init_score_ms"],
+                 "kernel": "fit_const_closed, fit_queue, fit_score_warp / fit_score_queue kernels, init round of the "
+                           "refined fit (three tile-size classes)", "ms": dbd["init_score_ms"],
                  "ms_samples": [round(v, 4) for v in dbd["init_score_samples"]],
                  "launches": dbd["init_score_launches"], "peak_source": fp32_src}
     n_cand = int(sum(len(p) for p in dev_cl))

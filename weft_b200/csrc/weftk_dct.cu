@@ -9,7 +9,7 @@
 // as a matrix product with the DCT-II basis A[k][x] = c_k cos(pi (2x + 1) k / (2n)).
 // Bound: latency (two CTAs a SM, a fill of the chip once: the gather, the basis and the image's pixels are
 // each asked for in batches) and instruction issue; the float64 pipes are 9 % busy.  A 1024 x 1024 picture
-// with its tiles of 8 to 64 px takes 38 us, 4:2:0, and took 191 with a CTA per tile, one output of a pass
+// with its tiles of 8 to 64 px takes 41 us, 4:2:0, and took 191 with a CTA per tile, one output of a pass
 // per thread, the basis read from memory and a launch per side.
 //
 // Resize: Pillow's ImagingResample for 8-bit images.  A sample's taps (bounds, float64 triangle
